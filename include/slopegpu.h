@@ -155,6 +155,18 @@ int sg_force_dev(const sg_mesh *mesh, const double *S, int32_t s_rows, double *F
  * zeroed and written.  3D, n_p = 10 only (SG_ERR_ARG otherwise). */
 int sg_residual_dev(const sg_mesh *mesh, const double *U, const double *c_bar, const double *sin_phi,
                     const double *shear, const double *lame, uint8_t *branch, double *F, void *stream);
+/* (a4 + a5 + a1/a2 + a6 fused) the whole element response at a displacement in one pass over
+ * the points: Davis reduction of c0, phi, psi at lambda ('A', 'B', 'C') into c_bar, sin_phi
+ * (written), strain, return mapping and internal force F (dim x n_n, zeroed and written), i.e.
+ * CONSTITUTIVE.build_F_all / build_F_and_DS_all (CONSTITUTIVE.m:178-285, 309-348, 466-485).
+ * c0 = NULL: no reduction, c_bar and sin_phi are read.  DS (optional) receives the tangent,
+ * E and S (optional; on tetrahedra only together with DS) strain and stress, branch (optional)
+ * the branch ids.  P2 triangles (n_p = 6) and tetrahedra (n_p = 10), n_q <= 16 (SG_ERR_ARG
+ * otherwise). */
+int sg_element_response_dev(const sg_mesh *mesh, const double *U, const double *c0, const double *phi,
+                            const double *psi, double lambda, char davis_type, double *c_bar, double *sin_phi,
+                            const double *shear, const double *lame, double *E, double *S, double *DS,
+                            uint8_t *branch, double *F, void *stream);
 /* (b3) K_t = sum_e B'(w DS)B into the block pattern (values zeroed first) */
 int sg_assemble_bsr_dev(const sg_mesh *mesh, const double *DS, double *K, void *stream);
 /* DS_elast of CONSTITUTIVE.m:413-422 per point (n_strain^2 x n_int) */

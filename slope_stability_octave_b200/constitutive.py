@@ -129,36 +129,43 @@ class CONSTITUTIVE:
 
     def build_F(self, out=None):
         with _Timer(self.profiler, "CONSTITUTIVE.build_F"):
-            F = self.F if out is None else out
-            self.m.force(self.S, self.s_rows, F)
-        return F.clone() if out is None else F
+            if out is None:
+                self.F = out = torch.empty_like(self.F)     # earlier results stay with their holders
+            self.m.force(self.S, self.s_rows, out)
+        return out
 
-    def _residual(self, U):
-        """F(U) at the current reduction: one fused kernel (strain, stress-only return mapping,
-        internal force) on P2 tetrahedra, the three steps otherwise.  The fused path leaves
-        E and S unset."""
-        if not self.m.fused_residual:
-            self.constitutive_problem_stress(U)
+    def _response(self, U, lam, tangent):
+        """F(U), with S and DS when ``tangent``, at the reduction factor ``lam`` (None: the
+        current one): one fused kernel on P2 elements, the separate steps otherwise.  The
+        stress-only path leaves E and S unset in 3D."""
+        m = self.m
+        if not m.fused_response:
+            if lam is not None:
+                self.reduction(lam)
+            (self.constitutive_problem_stress_tangent if tangent else self.constitutive_problem_stress)(U)
             return self.build_F()
-        with _Timer(self.profiler, "CONSTITUTIVE.residual"):
-            self.m.residual(U, self.c_bar, self.sin_phi, self.shear, self.lame, self.branch, self.F)
-        return self.F.clone()
+        with _Timer(self.profiler, "CONSTITUTIVE.tangent" if tangent else "CONSTITUTIVE.residual"):
+            F = torch.empty_like(self.F)
+            keep = tangent or self.dim == 2
+            m.response(U, None if lam is None else (self.c0, self.phi, self.psi, lam, self.Davis_type), self.c_bar,
+                       self.sin_phi, self.shear, self.lame, self.E if keep else None, self.S if keep else None,
+                       self.DS if tangent else None, self.branch, F)
+            self.F = F
+            if lam is not None:
+                self.lambda_ = float(lam)
+        return F
 
     def build_F_all(self, lam, U):
-        self.reduction(lam)
-        return self._residual(U)
+        return self._response(U, lam, False)
 
     def build_F_reduced(self, U):
-        return self._residual(U)
+        return self._response(U, None, False)
 
     def build_F_and_DS_all(self, lam, U):
-        self.reduction(lam)
-        self.constitutive_problem_stress_tangent(U)
-        return self.build_F()
+        return self._response(U, lam, True)
 
     def build_F_and_DS_reduced(self, U):
-        self.constitutive_problem_stress_tangent(U)
-        return self.build_F()
+        return self._response(U, None, True)
 
     # -------------------------------------------------------------- stiffness
     def init_K_r_pattern(self, Q=None):

@@ -54,64 +54,84 @@ __device__ __forceinline__ void sylvester(const double tsq[6], const double t[6]
     for (int i = 3; i < 6; ++i) P[i] = scale * (tsq[i] - bc_sum * t[i]);
 }
 
-// Quantities shared by every branch: the stress-representation strain t, t^2, I1, the
-// ordered principal strains e1 >= e2 >= e3 and the trial yield value.
+// Quantities shared by every branch: the stress-representation strain t, its invariants, and
+// (plastic points) t^2, the ordered principal strains e1 >= e2 >= e3 and the trial yield value.
 struct MC3Pre {
     double t[6], tsq[6], I1, e1, e2, e3, f_tr;
+    double I2, Qv;       // closed form of the principal strains: e = I1 / 3 + 2 sqrt(Qv) cos(.)
 };
 
-__device__ __forceinline__ void mc3d_prefix(const double E[6], double c_bar, double sin_phi, double shear,
-                                            double lame, MC3Pre &q) {
-    const double sp = sin_phi;
-    double *t = q.t, *tsq = q.tsq;
+__device__ __forceinline__ void mc3d_invariants(const double E[6], MC3Pre &q) {
+    double *t = q.t;
     t[0] = E[0];
     t[1] = E[1];
     t[2] = E[2];
     t[3] = 0.5 * E[3];
     t[4] = 0.5 * E[4];
     t[5] = 0.5 * E[5];
+    q.I1 = t[0] + t[1] + t[2];
+    q.I2 = t[0] * t[1] + t[0] * t[2] + t[1] * t[2] - t[3] * t[3] - t[4] * t[4] - t[5] * t[5];
+    const double Qv = (q.I1 * q.I1 - 3.0 * q.I2) * (1.0 / 9.0);
+    q.Qv = Qv < 0.0 ? 0.0 : Qv;
+}
+
+// True only where the trial yield value is negative beyond any rounding of it, decided
+// without the principal strains.  Over the Lode angle the deviatoric part of
+// (1 + s) e1 - (1 - s) e3 is at most 2 sqrt(Q) sqrt(3 + s^2) <= 2 sqrt(Q) (sqrt(3) + s^2 / (2 sqrt(3))),
+// so a point with 4 G sqrt(Q) (..) below what volume and cohesion leave, less 1e-12 of the
+// terms' size, is elastic by the reference's test as well (whose rounding is about 1e-15 of
+// them).  NaN and infinities fail the comparison and take the full path.  On the slopes
+// three quarters and more of the points are elastic and lie together, so whole warps leave
+// before the square root, acos, sines, divides and branch tests.
+__device__ __forceinline__ bool mc3d_surely_elastic(const MC3Pre &q, double c_bar, double sp, double shear,
+                                                    double lame) {
+    const double dev = 4.0 * shear * (1.7320508075688774 + 0.28867513459481293 * sp * sp);
+    const double vol = sp * q.I1 * ((4.0 / 3.0) * shear + 2.0 * lame);
+    const double left = (c_bar - vol) - 1e-12 * (fabs(c_bar) + 2.0 * (shear + fabs(lame)) * fabs(q.I1));
+    return left > 0.0 && dev * dev * q.Qv < left * left * (1.0 - 1e-11) && shear > 0.0 && fabs(sp) <= 1.0 &&
+           fabs(c_bar) < 1e300;
+}
+
+__device__ __forceinline__ void mc3d_principal(double c_bar, double sp, double shear, double lame, MC3Pre &q) {
+    const double *t = q.t, I1 = q.I1, I2 = q.I2;
+    double *tsq = q.tsq;
     tsq[0] = t[0] * t[0] + t[3] * t[3] + t[5] * t[5];
     tsq[1] = t[1] * t[1] + t[3] * t[3] + t[4] * t[4];
     tsq[2] = t[2] * t[2] + t[4] * t[4] + t[5] * t[5];
     tsq[3] = t[0] * t[3] + t[1] * t[3] + t[4] * t[5];
     tsq[4] = t[3] * t[5] + t[1] * t[4] + t[2] * t[4];
     tsq[5] = t[0] * t[5] + t[3] * t[4] + t[2] * t[5];
-    const double I1 = t[0] + t[1] + t[2];
-    const double I2 = t[0] * t[1] + t[0] * t[2] + t[1] * t[2] - t[3] * t[3] - t[4] * t[4] - t[5] * t[5];
     const double I3 = t[0] * t[1] * t[2] - t[2] * t[3] * t[3] - t[1] * t[5] * t[5] - t[0] * t[4] * t[4] +
                       2.0 * t[3] * t[4] * t[5];
-    double Qv = (I1 * I1 - 3.0 * I2) / 9.0;
-    if (Qv < 0.0) Qv = 0.0;
-    const double Rv = (-2.0 * I1 * I1 * I1 + 9.0 * I1 * I2 - 27.0 * I3) / 54.0;
-    const double rq = sqrt(Qv);
+    const double Rv = (-2.0 * I1 * I1 * I1 + 9.0 * I1 * I2 - 27.0 * I3) * (1.0 / 54.0);
+    const double rq = sqrt(q.Qv);
     double theta = 0.0;
-    if (!(Qv < 1e-30)) {
-        double c = Rv / (rq * Qv);
+    if (!(q.Qv < 1e-30)) {
+        double c = Rv / (rq * q.Qv);
         c = fmin(fmax(c, -1.0), 1.0);
-        theta = acos(c) / 3.0;
+        theta = acos(c) * (1.0 / 3.0);
     }
-    const double two_pi_3 = 2.0 * 3.14159265358979323846 / 3.0;
-    const double e1 = -2.0 * rq * cos(theta + two_pi_3) + I1 / 3.0;
-    const double e2 = -2.0 * rq * cos(theta - two_pi_3) + I1 / 3.0;
-    const double e3 = -2.0 * rq * cos(theta) + I1 / 3.0;
-
-    const double f_tr = 2.0 * shear * ((1.0 + sp) * e1 - (1.0 - sp) * e3) + 2.0 * lame * sp * I1 - c_bar;
-    q.I1 = I1;
-    q.e1 = e1;
-    q.e2 = e2;
-    q.e3 = e3;
-    q.f_tr = f_tr;
+    // cos(theta +- 2 pi / 3) = -cos(theta) / 2 -+ sqrt(3) / 2 sin(theta)
+    double sn, cs;
+    sincos(theta, &sn, &cs);
+    const double m = I1 * (1.0 / 3.0), a = rq * cs, b = 1.7320508075688772 * rq * sn;
+    q.e1 = (a + b) + m;
+    q.e2 = (a - b) + m;
+    q.e3 = -2.0 * a + m;
+    q.f_tr = 2.0 * shear * ((1.0 + sp) * q.e1 - (1.0 - sp) * q.e3) + 2.0 * lame * sp * I1 - c_bar;
 }
 
 // The branch the reference's kernel takes for this point (its tests, in its order).
 __device__ __forceinline__ int mc3d_classify(const MC3Pre &q, double c_bar, double sp, double shear, double lame) {
     if (q.f_tr <= 0.0) return BR_ELASTIC;
     const double e1 = q.e1, e2 = q.e2, e3 = q.e3, I1 = q.I1;
-    const double g_sl = (e1 - e2) / (1.0 + sp);
-    const double g_sr = (e2 - e3) / (1.0 - sp);
     const double den_s = 4.0 * lame * sp * sp + 4.0 * shear * (1.0 + sp * sp);
     const double dl_s = q.f_tr / den_s;
-    if (dl_s <= g_sl && dl_s <= g_sr) return BR_SMOOTH;
+    // dl_s <= g_sl and dl_s <= g_sr with the denominators 1 +- sp multiplied out
+    if (fabs(sp) < 1.0 && dl_s * (1.0 + sp) <= e1 - e2 && dl_s * (1.0 - sp) <= e2 - e3) return BR_SMOOTH;
+    const double g_sl = (e1 - e2) / (1.0 + sp);
+    const double g_sr = (e2 - e3) / (1.0 - sp);
+    if (fabs(sp) >= 1.0 && dl_s <= g_sl && dl_s <= g_sr) return BR_SMOOTH;
     if (g_sl < g_sr) {
         const double den_l = 4.0 * lame * sp * sp + shear * (1.0 + sp) * (1.0 + sp) +
                              2.0 * shear * (1.0 - sp) * (1.0 - sp);
@@ -158,9 +178,10 @@ __device__ __forceinline__ void mc3d_finish(const MC3Pre &q, int br, double c_ba
     if (br == BR_SMOOTH) {
         const double den_s = 4.0 * lame * sp * sp + 4.0 * shear * (1.0 + sp * sp);
         const double dl_s = f_tr / den_s;
-        const double k1 = 1.0 / ((e1 - e2) * (e1 - e3));
-        const double k2 = 1.0 / ((e2 - e1) * (e2 - e3));
-        const double k3 = 1.0 / ((e3 - e1) * (e3 - e2));
+        // 1 / ((e1 - e2)(e1 - e3)) and its cyclic companions from one divide
+        const double b1 = e2 - e3, b2 = e1 - e3, b3 = e1 - e2;
+        const double kk = 1.0 / (b1 * b2 * b3);
+        const double k1 = kk * b1, k2 = -kk * b2, k3 = kk * b3;
         double P1[6], P2[6], P3[6];
         sylvester(tsq, t, e2 + e3, e2 * e3, k1, P1);
         sylvester(tsq, t, e1 + e3, e1 * e3, k2, P2);
@@ -175,24 +196,27 @@ __device__ __forceinline__ void mc3d_finish(const MC3Pre &q, int br, double c_ba
 #pragma unroll
             for (int i = 0; i < 6; ++i)
                 n[i] = 2.0 * shear * ((1.0 + sp) * P1[i] - (1.0 - sp) * P3[i]) + 2.0 * lame * sp * unit3(i);
-            const double a1 = 2.0 * e1 - e2 - e3, b1 = e2 - e3;
-            const double a2 = 2.0 * e2 - e1 - e3, b2 = e1 - e3;
-            const double a3 = 2.0 * e3 - e1 - e2, b3 = e1 - e2;
+            // sum_m s_m dP_m/dE with Miehe's dP_m/dE = k_m (dT^2/dE - (e_n + e_o) Id
+            // - (2 e_m - e_n - e_o) P_m P_m' - (e_n - e_o)(P_n P_n' - P_o P_o')), the terms
+            // collected by tensor: nine operations per entry instead of 25
+            const double w1 = s1 * k1, w2 = s2 * k2, w3 = s3 * k3;
+            const double cd = w1 + w2 + w3;
+            const double ch = -(w1 * (e2 + e3) + w2 * (e1 + e3) + w3 * (e1 + e2));
+            const double c1 = 2.0 * shear - (w1 * (b2 + b3) + w2 * b2 + w3 * b3);
+            const double c2 = 2.0 * shear - (w1 * b1 + w2 * (b1 - b3) - w3 * b3);
+            const double c3 = 2.0 * shear + (w1 * b1 + w2 * b2 + w3 * (b1 + b2));
             const double inv_den = 1.0 / den_s;
 #pragma unroll
-            for (int j = 0; j < 6; ++j)
+            for (int j = 0; j < 6; ++j) {
+                const double p1 = c1 * P1[j], p2 = c2 * P2[j], p3 = c3 * P3[j], nj = n[j] * inv_den;
 #pragma unroll
                 for (int i = 0; i <= j; ++i) {
-                    const double hi = half_id(i, j), d = dsq(t, i, j);
-                    const double q11 = P1[i] * P1[j], q22 = P2[i] * P2[j], q33 = P3[i] * P3[j];
-                    const double d1 = k1 * (d - hi * (e2 + e3) - a1 * q11 - b1 * (q22 - q33));
-                    const double d2 = k2 * (d - hi * (e1 + e3) - a2 * q22 - b2 * (q11 - q33));
-                    const double d3 = k3 * (d - hi * (e1 + e2) - a3 * q33 - b3 * (q11 - q22));
-                    const double v = s1 * d1 + s2 * d2 + s3 * d3 + lame * unit3(i) * unit3(j) +
-                                     2.0 * shear * (q11 + q22 + q33) - n[i] * n[j] * inv_den;
+                    const double v = cd * dsq(t, i, j) + ch * half_id(i, j) + lame * unit3(i) * unit3(j) +
+                                     P1[i] * p1 + P2[i] * p2 + P3[i] * p3 - n[i] * nj;
                     ds[i + 6 * j] = v;
                     ds[j + 6 * i] = v;
                 }
+            }
         }
         return;
     }
@@ -293,8 +317,12 @@ template <bool WANT_DS>
 __device__ __forceinline__ int mc3d_point(const double E[6], double c_bar, double sin_phi,
                                           double shear, double lame, double S[6], double *ds) {
     MC3Pre q;
-    mc3d_prefix(E, c_bar, sin_phi, shear, lame, q);
-    const int br = mc3d_classify(q, c_bar, sin_phi, shear, lame);
+    mc3d_invariants(E, q);
+    int br = BR_ELASTIC;
+    if (!mc3d_surely_elastic(q, c_bar, sin_phi, shear, lame)) {
+        mc3d_principal(c_bar, sin_phi, shear, lame, q);
+        br = mc3d_classify(q, c_bar, sin_phi, shear, lame);
+    }
     mc3d_finish<WANT_DS>(q, br, c_bar, sin_phi, shear, lame, S, ds);
     return br;
 }
@@ -521,27 +549,41 @@ __device__ __forceinline__ double potential2d(const double E[3], double c_bar, d
 
 __device__ __forceinline__ void davis_reduce(double c0, double phi, double psi, double lambda, char type,
                                              double &c_bar, double &sin_phi) {
-    double beta, c_l, phi_l;
+    // u = tan of the reduced friction angle.  The reference takes cos and sin of arctangents;
+    // with t = tan(f), f in (-pi/2, pi/2): cos f = 1 / sqrt(1 + t^2), sin f = t cos f.
+    double beta, c_l, u;
+    const double inv = 1.0 / lambda;
     if (type == 'A') {
-        beta = cos(phi) * cos(psi) / (1.0 - sin(phi) * sin(psi));
-        c_l = beta * c0 / lambda;
-        phi_l = atan(beta * tan(phi) / lambda);
+        double sf, cf, ss = 0.0, cs = 1.0;
+        sincos(phi, &sf, &cf);
+        if (psi != 0.0) sincos(psi, &ss, &cs);
+        beta = cf * cs / (1.0 - sf * ss);
+        c_l = beta * (c0 * inv);
+        u = beta * (tan(phi) * inv);
     } else if (type == 'B') {
-        const double c1 = c0 / lambda;
-        const double f1 = atan(tan(phi) / lambda);
-        const double s1 = atan(tan(psi) / lambda);
-        beta = cos(f1) * cos(s1) / (1.0 - sin(f1) * sin(s1));
-        c_l = beta * c1;
-        phi_l = atan(beta * tan(f1));
+        const double tf = tan(phi) * inv, rf = rsqrt(1.0 + tf * tf);
+        beta = rf;
+        if (psi != 0.0) {   // psi = 0 in most scripts (NaN takes this path too)
+            const double ts = tan(psi) * inv, rs = rsqrt(1.0 + ts * ts);
+            beta = rf * rs / (1.0 - (tf * rf) * (ts * rs));
+        }
+        c_l = beta * (c0 * inv);
+        u = beta * tf;
     } else {
-        const double c1 = c0 / lambda;
-        const double f1 = atan(tan(phi) / lambda);
-        beta = (f1 > psi) ? cos(f1) * cos(psi) / (1.0 - sin(f1) * sin(psi)) : 1.0;
-        c_l = beta * c1;
-        phi_l = atan(beta * tan(f1));
+        const double tf = tan(phi) * inv;
+        beta = 1.0;
+        if (atan(tf) > psi) {
+            const double rf = rsqrt(1.0 + tf * tf);
+            double ss, cs;
+            sincos(psi, &ss, &cs);
+            beta = rf * cs / (1.0 - (tf * rf) * ss);
+        }
+        c_l = beta * (c0 * inv);
+        u = beta * tf;
     }
-    c_bar = 2.0 * c_l * cos(phi_l);
-    sin_phi = sin(phi_l);
+    const double r = rsqrt(1.0 + u * u);
+    c_bar = 2.0 * c_l * r;
+    sin_phi = u * r;
 }
 
 }  // namespace sg

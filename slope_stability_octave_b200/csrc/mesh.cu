@@ -22,6 +22,7 @@
 #include <new>
 
 #include "mesh.h"
+#include "p2tet.cuh"
 #include "sg_common.cuh"
 
 namespace sg {
@@ -192,6 +193,7 @@ static int mesh_build(sg_mesh *m, const int32_t *elem, const double *D1, const d
     if (!rc) rc = upload(&m->d_w, W, (size_t)n_int);
     if (!rc) rc = upload(&m->d_mask, mask.data(), mask.size());
     if (!rc) rc = upload(&m->d_pair_blk, pair.data(), pair.size());
+    if (!rc) rc = p2tet_factor(m, D1, D2, D3);
     return rc;
 }
 
@@ -269,6 +271,7 @@ extern "C" int sg_mesh_destroy(sg_mesh *m) {
     cudaFree(m->d_contrib_ptr);
     cudaFree(m->d_contrib);
     cudaFree(m->d_ke);
+    cudaFree(m->d_gxi);
     cudaFree(m->d_ref2bsr);
     cudaSetDevice(cur);
     delete m;

@@ -44,6 +44,10 @@ struct sg_mesh {
     int32_t *d_contrib_ptr = nullptr; // n_blocks + 1
     uint32_t *d_contrib = nullptr;    // n_e * np * np entries: e * 55 + s | transposed << 31
     double *d_ke = nullptr;           // n_e * 55 * 10: element upper node blocks, 9 values + 1 pad (allocated on first use)
+    // factored gradients of isoparametric P2 tetrahedra (p2tet.cuh): G_1, G_2, G_3 of an element's
+    // points as [e][9][q], and the rule's barycentric coordinates; null when they do not apply
+    double *d_gxi = nullptr;
+    double rule[16][4] = {};
     int device = 0;
 };
 

@@ -134,6 +134,20 @@ class DeviceMesh:
         """The fused stress-only residual kernel covers P2 tetrahedra."""
         return self.dim == 3 and self.mesh.elem.shape[0] == 10
 
+    @property
+    def fused_response(self):
+        """The fused element response (reduction, strain, return mapping, force in one kernel)
+        covers P2 triangles and tetrahedra."""
+        return (self.dim, self.mesh.elem.shape[0]) in ((3, 10), (2, 6)) and self.n_q <= 16
+
+    def response(self, U, reduce, c_bar, sin_phi, shear, lame, E, S, DS, branch, F):
+        """F at U, with the tangent when DS is given; ``reduce`` = (c0, phi, psi, lambda,
+        Davis type) reduces the strength on the way (c_bar, sin_phi written), None reads it."""
+        c0, phi, psi, lam, davis = reduce if reduce is not None else (None, None, None, 1.0, "B")
+        _lib.call("sg_element_response_dev", self.handle, ptr(U), ptr(c0), ptr(phi), ptr(psi), float(lam),
+                  davis.encode(), ptr(c_bar), ptr(sin_phi), ptr(shear), ptr(lame), ptr(E), ptr(S), ptr(DS),
+                  ptr(branch), ptr(F), cur_stream())
+
     def residual(self, U, c_bar, sin_phi, shear, lame, branch, F):
         _lib.call("sg_residual_dev", self.handle, ptr(U), ptr(c_bar), ptr(sin_phi), ptr(shear), ptr(lame),
                   ptr(branch) if branch is not None else None, ptr(F), cur_stream())
