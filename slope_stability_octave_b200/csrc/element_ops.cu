@@ -19,6 +19,7 @@
 #include "instr.cuh"
 #include "mc_point.cuh"
 #include "mesh.h"
+#include "p2tet.cuh"
 #include "sg_common.cuh"
 
 namespace sg {
@@ -174,15 +175,15 @@ __global__ void __launch_bounds__(128) k_assemble_bsr(const int32_t *__restrict_
 //       sum_q w_q B_q' sym(D_q) B_q, with the element's D, gradients and weights staged in
 //       shared memory once; D B is formed once per (point, column) and shared by the blocks;
 //       diagonal blocks are computed on and above their diagonal and mirrored;
-//   k_gather_blocks3        per BSR block, the sum of its element contributions in element
-//       order (the transpose of an upper block for the lower ones), written as K_t, or
+//   k_gather_upper          per BSR block on or above the diagonal, the sum of its element
+//       contributions in element order, written with its transpose as K_t, or
 //       blended into K_r = r K_el + (1 - r) K_t with identity on Dirichlet rows/columns
 //       (the k_kr_blend epilogue; K_el and K_t being exactly symmetric, its averaging with the
 //       transposed block is the identity).
 // sym(D) = (D + D')/2 is what the reference's symmetrisation of K_r applies to its unsymmetric
 // sums (CONSTITUTIVE.m:515-532): B' sym(D) B = sym(B' D B).
 constexpr int KE_EPB = 8, KE_TPE = 18;   // elements per CTA, threads per element (one per chunk)
-constexpr int KE_PITCH = 10;             // doubles per stored element block (9 + 1: 16-byte aligned)
+constexpr int KE_PITCH = 9;              // doubles per stored element block
 
 // The 18 chunks of an element's upper node blocks: node j and up to 4 row nodes i0 .. i0+3
 // (i <= j); chunk c owns blocks (i, j) for i in [i0, min(i0 + 4, j + 1)).
@@ -394,87 +395,95 @@ __global__ void __launch_bounds__(KE_EPB * KE_TPE, 2) k_element_blocks_p2tet_bul
     }
 }
 
-// A warp sums the contributions of 32 consecutive blocks (a lane per block, its element
-// blocks read as five 16-byte words), then writes the 32 results as one contiguous run through
-// shared memory (and reads K_el for the blend the same way).
-constexpr int KG_WARPS = 8;
+// Sums the contributions of every block on or above the diagonal (an "item") and writes the
+// block and its transpose.  Nine lanes per item, three items per warp step and KG_STEP steps
+// whose loads are issued before any is added: an item's record and source list are broadcast
+// loads, a contribution one contiguous 72-byte run, read transposed where the element has the
+// pair the other way round.  The mesh lists the items of a window in descending number of
+// contributions, so the items of a step need the same number of loads; each item's
+// contributions are added in list (element) order.
+//
+// What bounds it: memory latency, at half of the DRAM rate (element blocks once, 3,960 bytes an
+// element; forming the lower blocks from the upper ones reads them once instead of twice; K_el and
+// K_r once each).  Two dependent loads reach a value (record, element block); a CTA per
+// 48 items, so that the hardware spreads the items with many contributions (a stride over the
+// sorted windows put them on the same CTAs: 106 against 147 us).  Measured on B200, layered
+// slope (14.7M items, 28.3M blocks) 3.23 -> 1.61 ms, 446k-point slope 183 -> 98 us, both against
+// a lane per block over all blocks; one or three steps per warp 1.91 / 1.66 ms, the
+// contributions of a batch staged in shared memory by cp.async 2.65 ms.
+constexpr int KG_THREADS = 256, KG_STEP = 2, KG_LOADS = 4;
+
 template <bool BLEND>
-__global__ void __launch_bounds__(KG_WARPS * 32) k_gather_blocks3(int64_t n_blocks, const int32_t *__restrict__ cptr,
-                                                                  const uint32_t *__restrict__ contrib,
-                                                                  const double *__restrict__ Ke,
-                                                                  const int32_t *__restrict__ row_of,
-                                                                  const int32_t *__restrict__ col,
-                                                                  const double *__restrict__ mask, double r,
-                                                                  const double *__restrict__ Kel,
-                                                                  double *__restrict__ Kout) {
-    __shared__ double sOut[KG_WARPS][32 * 9];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double *so = sOut[warp];
-    const int64_t stride = (int64_t)gridDim.x * KG_WARPS * 32;
-    for (int64_t base = ((int64_t)blockIdx.x * KG_WARPS + warp) * 32; base < n_blocks; base += stride) {
-        const int64_t p = base + lane;
-        double acc[9];
+__global__ void __launch_bounds__(KG_THREADS, 4) k_gather_upper(int64_t n_items, const int4 *__restrict__ items,
+                                                                const uint32_t *__restrict__ src,
+                                                                const double *__restrict__ Ke, double r,
+                                                                const double *__restrict__ Kel,
+                                                                double *__restrict__ Kout) {
+    const int lane = threadIdx.x & 31, sub = lane / 9, k = lane - sub * 9, ka = k / 3, kb = k - ka * 3, kt = kb * 3 + ka;
+    const int64_t stride = (int64_t)gridDim.x * (KG_THREADS / 32) * (3 * KG_STEP);
+    if (sub == 3) return;
+    auto value = [&](uint32_t s) { return __ldg(Ke + (int64_t)(s & 0x7fffffffu) * 9 + ((s >> 31) ? kt : k)); };
+    for (int64_t base = ((int64_t)blockIdx.x * (KG_THREADS / 32) + (threadIdx.x >> 5)) * (3 * KG_STEP) + sub;
+         base < n_items; base += stride) {
+        int4 it[KG_STEP], s4[KG_STEP]; // block, transposed block, further contributions, count | free << 24; first four
+        double x[KG_STEP][KG_LOADS], e0[KG_STEP], e1[KG_STEP];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) acc[k] = 0.0;
-        if (p < n_blocks) {
-            // contributions in list order, two in flight (both index and block loads issued
-            // before either is added)
-            auto add = [&](uint32_t src, const double *x) {
-                if (src >> 31) {
+        for (int u = 0; u < KG_STEP; ++u) {
+            const bool in = base + 3 * u < n_items;
+            it[u] = in ? __ldg(items + 2 * (base + 3 * u)) : make_int4(-1, -1, 0, 0);
+            s4[u] = in ? __ldg(items + 2 * (base + 3 * u) + 1) : make_int4(0, 0, 0, 0);
+        }
 #pragma unroll
-                    for (int a = 0; a < 3; ++a)
+        for (int u = 0; u < KG_STEP; ++u) {
+            const int n = it[u].w & 0xffffff;
+            const uint32_t s[KG_LOADS] = {(uint32_t)s4[u].x, (uint32_t)s4[u].y, (uint32_t)s4[u].z, (uint32_t)s4[u].w};
 #pragma unroll
-                        for (int b = 0; b < 3; ++b) acc[a * 3 + b] += x[b * 3 + a];
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 9; ++k) acc[k] += x[k];
-                }
-            };
-            auto fetch = [&](uint32_t src, double *x) {
-                const double2 *v = reinterpret_cast<const double2 *>(Ke + (int64_t)(src & 0x7fffffffu) * KE_PITCH);
-#pragma unroll
-                for (int h = 0; h < 5; ++h) {
-                    const double2 t = __ldg(v + h);
-                    x[2 * h] = t.x;
-                    x[2 * h + 1] = t.y;
-                }
-            };
-            const int32_t l1 = cptr[p + 1];
-            int32_t l = cptr[p];
-            for (; l + 1 < l1; l += 2) {
-                const uint32_t s0 = contrib[l], s1 = contrib[l + 1];
-                double x0[10], x1[10];
-                fetch(s0, x0);
-                fetch(s1, x1);
-                add(s0, x0);
-                add(s1, x1);
-            }
-            if (l < l1) {
-                const uint32_t s0 = contrib[l];
-                double x0[10];
-                fetch(s0, x0);
-                add(s0, x0);
+            for (int l = 0; l < KG_LOADS; ++l) x[u][l] = l < n ? value(s[l]) : 0.0;
+            e0[u] = e1[u] = 0.0;
+            if (BLEND && Kel && it[u].x >= 0) {
+                e0[u] = __ldg(Kel + (int64_t)it[u].x * 9 + k);
+                e1[u] = __ldg(Kel + (int64_t)it[u].y * 9 + kt);
             }
         }
 #pragma unroll
-        for (int k = 0; k < 9; ++k) so[lane * 9 + k] = acc[k];
-        __syncwarp();
-        const int cnt = (int)(n_blocks - base < 32 ? n_blocks - base : 32);
-        for (int idx = lane; idx < cnt * 9; idx += 32) {
-            const int pl = idx / 9, k = idx - pl * 9;
-            const int64_t o = base * 9 + idx;
-            double v = so[idx];
+        for (int u = 0; u < KG_STEP; ++u) {
+            if (it[u].x < 0) continue;
+            const int n = it[u].w & 0xffffff;
+            double v = x[u][0];
+#pragma unroll
+            for (int l = 1; l < KG_LOADS; ++l) v += x[u][l];
+            const uint32_t *more = src + it[u].z;
+            int left = n - KG_LOADS;
+            for (; left >= 4; left -= 4, more += 4) {
+                uint32_t s[4];
+                double y[4];
+#pragma unroll
+                for (int h = 0; h < 4; ++h) s[h] = __ldg(more + h);
+#pragma unroll
+                for (int h = 0; h < 4; ++h) y[h] = value(s[h]);
+#pragma unroll
+                for (int h = 0; h < 4; ++h) v += y[h];
+            }
+            for (; left > 0; --left, ++more) v += value(__ldg(more));
+            double a = v, t = v;
             if (BLEND) {
-                const int64_t pb = base + pl, I = row_of[pb], J = col[pb];
-                const int a = k / 3, b = k - a * 3;
-                const bool free = mask[I * 3 + a] != 0.0 && mask[J * 3 + b] != 0.0;
-                const double el = Kel ? Kel[o] : 0.0;
-                v = free ? r * el + (1.0 - r) * v : ((I == J && a == b) ? 1.0 : 0.0);
+                const bool free = (it[u].w >> (24 + ka) & 1) && (it[u].w >> (27 + kb) & 1);
+                const double unit = it[u].x == it[u].y && ka == kb ? 1.0 : 0.0;
+                a = free ? r * e0[u] + (1.0 - r) * v : unit;
+                t = free ? r * e1[u] + (1.0 - r) * v : unit;
             }
-            Kout[o] = v;
+            Kout[(int64_t)it[u].x * 9 + k] = a;
+            if (it[u].x != it[u].y) Kout[(int64_t)it[u].y * 9 + kt] = t;
         }
-        __syncwarp();
     }
+}
+
+static int gather_blocks(const sg_mesh *m, bool blend, double r, const double *Kel, double *K, cudaStream_t st) {
+    const unsigned grid = grid_chunks(m->n_upper, KG_THREADS / 32 * 3 * KG_STEP);
+    if (blend) k_gather_upper<true><<<grid, KG_THREADS, 0, st>>>(m->n_upper, m->d_up_item, m->d_up_src, m->d_ke, r, Kel, K);
+    else k_gather_upper<false><<<grid, KG_THREADS, 0, st>>>(m->n_upper, m->d_up_item, m->d_up_src, m->d_ke, 0.0, nullptr, K);
+    SG_CUDA(cudaGetLastError());
+    return SG_OK;
 }
 
 // Element blocks of the deterministic path into m->d_ke (allocated on first use): the
@@ -482,6 +491,7 @@ __global__ void __launch_bounds__(KG_WARPS * 32) k_gather_blocks3(int64_t n_bloc
 // aligned and two stages fit in shared memory, else the plain-load kernel.
 static int element_blocks(sg_mesh *m, const double *DS, cudaStream_t st) {
     if (!m->d_ke) SG_CUDA(device_alloc(&m->d_ke, sizeof(double) * (size_t)m->n_e * 55 * KE_PITCH));
+    if (m->d_gxi && m->nq == P2T_REF_RULE) return p2tet_element_blocks(m, DS, m->d_ke, st);
     const int64_t batches = (m->n_e + KE_EPB - 1) / KE_EPB;
     const size_t stage = sizeof(double) * ((size_t)KE_EPB * m->nq * 66 + (size_t)((KE_EPB * m->nq + 1) & ~1));
     const size_t smem_bulk = 32 + 2 * stage;
@@ -515,7 +525,7 @@ static int element_blocks(sg_mesh *m, const double *DS, cudaStream_t st) {
     return SG_OK;
 }
 
-static bool deterministic_path(const sg_mesh *m) { return m->d_contrib && m->dim == 3 && m->np == 10; }
+static bool deterministic_path(const sg_mesh *m) { return m->d_up_src && m->dim == 3 && m->np == 10; }
 
 // DS_elast = 2 * shear * DEV + bulk * VOL with IOTA = [1;1;1; zeros(ns-3,1)] (CONSTITUTIVE.m:413-422).
 // For ns == 3 (2D) the reference's IOTA has three ones, so VOL is the all-ones 3x3 matrix;
@@ -615,11 +625,7 @@ extern "C" int sg_assemble_bsr_dev(const sg_mesh *m_, const double *DS, double *
     if (deterministic_path(m)) {
         const InstrToken tk = instr_begin(IK_ASSEMBLY, st);
         int rc = element_blocks(m, DS, st);
-        if (!rc) {
-            k_gather_blocks3<false><<<grid_for(m->bsr.n_blocks, KG_WARPS * 32, 8), KG_WARPS * 32, 0, st>>>(
-                m->bsr.n_blocks, m->d_contrib_ptr, m->d_contrib, m->d_ke, nullptr, nullptr, nullptr, 0.0, nullptr, K);
-            if (cudaGetLastError() != cudaSuccess) rc = set_error(SG_ERR_CUDA, "k_gather_blocks3 launch");
-        }
+        if (!rc) rc = gather_blocks(m, false, 0.0, nullptr, K, st);
         instr_end(tk, st);
         return rc;
     }
@@ -689,12 +695,7 @@ extern "C" int sg_assemble_kr_dev(sg_mesh *m, const double *DS, double r, const 
     if (deterministic_path(m)) {
         const InstrToken tk = instr_begin(IK_ASSEMBLY, st);
         int rc = element_blocks(m, DS, st);
-        if (!rc) {
-            k_gather_blocks3<true><<<grid_for(m->bsr.n_blocks, KG_WARPS * 32, 8), KG_WARPS * 32, 0, st>>>(
-                m->bsr.n_blocks, m->d_contrib_ptr, m->d_contrib, m->d_ke, m->bsr.d_row_of, m->bsr.d_col, m->d_mask, r,
-                Kel, Kr);
-            if (cudaGetLastError() != cudaSuccess) rc = set_error(SG_ERR_CUDA, "k_gather_blocks3 launch");
-        }
+        if (!rc) rc = gather_blocks(m, true, r, Kel, Kr, st);
         instr_end(tk, st);
         return rc;
     }

@@ -164,30 +164,74 @@ static int mesh_build(sg_mesh *m, const int32_t *elem, const double *D1, const d
     std::vector<double> mask(n_n * dim);
     for (int64_t d = 0; d < n_n * dim; ++d) mask[d] = m->Q[d] ? 1.0 : 0.0;
 
-    // contribution lists of the deterministic P2-tetrahedron assembly: block (node_i, node_j)
-    // of element e takes its upper slot s(min(i,j), max(i,j)), transposed when i > j; the lists
-    // are filled in element order, so every block sums its contributions in a fixed order
-    std::vector<int32_t> cptr;
-    std::vector<uint32_t> contrib;
+    // items of the deterministic P2-tetrahedron assembly: local pair (i, j), i <= j, of element e
+    // goes to block (node_i, node_j) when that lies on or above the diagonal, transposed to
+    // (node_j, node_i) otherwise; the lists are filled in element order, so every block sums
+    // its contributions in a fixed order
+    std::vector<int4> up_item;
+    std::vector<uint32_t> up_src;
     if (dim == 3 && np == 10 && n_e * 55 < ((int64_t)1 << 31)) {
-        cptr.assign(B.n_blocks + 1, 0);
-        for (size_t t = 0; t < pair.size(); ++t) cptr[pair[t] + 1]++;
-        for (int64_t p = 0; p < B.n_blocks; ++p) cptr[p + 1] += cptr[p];
-        std::vector<int32_t> fill(cptr.begin(), cptr.end() - 1);
-        contrib.resize(pair.size());
-        for (int64_t e = 0; e < n_e; ++e)
-            for (int i = 0; i < np; ++i)
-                for (int j = 0; j < np; ++j) {
-                    const int lo = std::min(i, j), hi = std::max(i, j);
-                    const uint32_t slot = (uint32_t)(lo * np - lo * (lo - 1) / 2 + (hi - lo));
-                    contrib[fill[pair[(e * np + i) * np + j]]++] =
-                        (uint32_t)(e * 55 + slot) | (i > j ? 0x80000000u : 0u);
-                }
+        std::vector<int32_t> count(B.n_blocks, 0);
+        auto each = [&](auto fn) {
+            for (int64_t e = 0; e < n_e; ++e)
+                for (int i = 0; i < np; ++i)
+                    for (int j = i; j < np; ++j) {
+                        const bool turn = m->elem[e * np + i] > m->elem[e * np + j];
+                        const int32_t p = pair[(e * np + (turn ? j : i)) * np + (turn ? i : j)];
+                        const uint32_t src = (uint32_t)(e * 55 + i * np - i * (i - 1) / 2 + (j - i));
+                        fn(p, src | (turn ? 0x80000000u : 0u));
+                        if (i < j && m->elem[e * np + i] == m->elem[e * np + j]) fn(p, src | 0x80000000u);
+                    }
+        };
+        each([&](int32_t p, uint32_t) { count[p]++; });
+        // items in windows of about a hundred rows, within a window in descending number of
+        // contributions: a warp's items then take the same number of loads, and what they write
+        // and read stays near in time
+        std::vector<int32_t> up;
+        up.reserve((size_t)(B.n_blocks / 2 + n_n));
+        for (int64_t v = 0; v < n_n; ++v)
+            for (int32_t p = B.row_ptr[v]; p < B.row_ptr[v + 1]; ++p)
+                if (B.col[p] >= v) up.push_back(p);
+        const int64_t nu = (int64_t)up.size(), window = 1536;
+#pragma omp parallel for schedule(static)
+        for (int64_t u0 = 0; u0 < nu; u0 += window)
+            std::stable_sort(up.begin() + u0, up.begin() + std::min(nu, u0 + window),
+                             [&](int32_t a, int32_t b) { return count[a] > count[b]; });
+        std::vector<int32_t> fill(B.n_blocks, 0);
+        int32_t at = 0;
+        for (int64_t u = 0; u < nu; ++u) {
+            fill[up[u]] = at;
+            at += std::max(count[up[u]] - 4, 0);
+        }
+        std::vector<int32_t> row_of(B.n_blocks);
+        for (int64_t v = 0; v < n_n; ++v)
+            for (int32_t p = B.row_ptr[v]; p < B.row_ptr[v + 1]; ++p) row_of[p] = (int32_t)v;
+        std::vector<int32_t> item(B.n_blocks, 0);
+        up_item.resize(2 * nu);
+#pragma omp parallel for schedule(static)
+        for (int64_t u = 0; u < nu; ++u) {
+            const int32_t p = up[u];
+            const int64_t v = row_of[p], w = B.col[p];
+            const int32_t *b0 = B.col.data() + B.row_ptr[w], *b1 = B.col.data() + B.row_ptr[w + 1];
+            int free = 0;
+            for (int c = 0; c < 3; ++c) free |= (m->Q[v * 3 + c] ? 1 << c : 0) | (m->Q[w * 3 + c] ? 8 << c : 0);
+            up_item[2 * u] = make_int4(p, (int)(std::lower_bound(b0, b1, (int32_t)v) - B.col.data()), fill[p],
+                                       count[p] | free << 24);
+            item[p] = (int32_t)u;
+        }
+        up_src.resize((size_t)std::max(at, 1));
+        std::fill(count.begin(), count.end(), 0);     // now: contributions placed
+        each([&](int32_t p, uint32_t src) {
+            const int32_t c = count[p]++;
+            if (c < 4) (&up_item[2 * (int64_t)item[p] + 1].x)[c] = (int)src;
+            else up_src[fill[p] + c - 4] = src;
+        });
+        m->n_upper = nu;
     }
 
     int rc = bsr_upload(B);
-    if (!rc && !contrib.empty()) rc = upload(&m->d_contrib_ptr, cptr.data(), cptr.size());
-    if (!rc && !contrib.empty()) rc = upload(&m->d_contrib, contrib.data(), contrib.size());
+    if (!rc && !up_src.empty()) rc = upload(&m->d_up_item, up_item.data(), up_item.size());
+    if (!rc && !up_src.empty()) rc = upload(&m->d_up_src, up_src.data(), up_src.size());
     if (!rc) rc = upload(&m->d_elem, m->elem.data(), (size_t)n_e * np);
     if (!rc) rc = upload(&m->d_dphi, dphi.data(), dphi.size());
     if (!rc) rc = upload(&m->d_w, W, (size_t)n_int);
@@ -268,9 +312,9 @@ extern "C" int sg_mesh_destroy(sg_mesh *m) {
     cudaFree(m->d_w);
     cudaFree(m->d_mask);
     cudaFree(m->d_pair_blk);
-    cudaFree(m->d_contrib_ptr);
-    cudaFree(m->d_contrib);
     cudaFree(m->d_ke);
+    cudaFree(m->d_up_item);
+    cudaFree(m->d_up_src);
     cudaFree(m->d_gxi);
     cudaFree(m->d_ref2bsr);
     cudaSetDevice(cur);

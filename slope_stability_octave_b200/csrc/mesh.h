@@ -39,11 +39,15 @@ struct sg_mesh {
     double *d_mask = nullptr;         // dim * n_n, 1 free / 0 Dirichlet
     int32_t *d_pair_blk = nullptr;    // n_e * np * np: block index of (node_i, node_j)
     int64_t *d_ref2bsr = nullptr;     // nnz_ref: value index of K(ref_I, ref_J) inside BSR values
-    // deterministic assembly of P2 tetrahedra: every BSR block's contributions (element e,
-    // upper node-block slot s of that element, transposed flag in bit 31) in element order
-    int32_t *d_contrib_ptr = nullptr; // n_blocks + 1
-    uint32_t *d_contrib = nullptr;    // n_e * np * np entries: e * 55 + s | transposed << 31
-    double *d_ke = nullptr;           // n_e * 55 * 10: element upper node blocks, 9 values + 1 pad (allocated on first use)
+    // deterministic assembly of P2 tetrahedra: an item of two int4 per block on or above the
+    // diagonal (block, transposed block, start of its further contributions, number of contributions |
+    // free components << 24: bits 0-2 of the row node, 3-5 of the column node; then its first
+    // four contributions), contributions in element order (element block e * 55 + s, bit 31 set
+    // when the element has the pair the other way round)
+    int64_t n_upper = 0;
+    int4 *d_up_item = nullptr;
+    uint32_t *d_up_src = nullptr;     // the contributions from the fifth on
+    double *d_ke = nullptr;           // n_e * 55 * 9: element upper node blocks (allocated on first use)
     // factored gradients of isoparametric P2 tetrahedra (p2tet.cuh): G_1, G_2, G_3 of an element's
     // points as [e][9][q], and the rule's barycentric coordinates; null when they do not apply
     double *d_gxi = nullptr;

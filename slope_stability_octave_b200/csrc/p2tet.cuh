@@ -32,4 +32,8 @@ int p2tet_factor(sg_mesh *m, const double *D1, const double *D2, const double *D
 // The reference's rule, for which the factored kernels are compiled.
 constexpr int P2T_REF_RULE = 11;
 
+// The element's 55 upper node blocks (9 values each, element-major) from DS into Ke, for
+// factored meshes with the reference's rule.
+int p2tet_element_blocks(const sg_mesh *m, const double *DS, double *Ke, cudaStream_t st);
+
 }  // namespace sg

@@ -89,3 +89,34 @@ def test_response_nan_and_infinite_displacement(cuda_device):
         cons.build_F_all(1.0, U)
         touched = cons.branch.view(mesh.n_e, 11)[0]
         assert (touched != 0).any()
+
+
+@pytest.mark.parametrize("cells,nq,numbering", [(1, 11, "reference"), (3, 11, "reference"), (2, 11, "swapped"),
+                                                (1, 1, "reference"), (2, 14, "reference")])
+def test_assembly_over_rules_and_numberings(cuda_device, cells, nq, numbering):
+    """K_t of tangents with all 36 entries free (sym(D) counts) against the element sums in
+    plain FP64, where the moments of the rule carry the blocks (11 points, factored gradients) and
+    where the direct sum does; a block adds up to some 24 x nq terms of alternating sign,
+    1e-12 of the largest entry as in the other assembly tests."""
+    mesh, dphi, w = problem(3, cells, nq, numbering)
+    dm = DeviceMesh(mesh, dphi, w, nq)
+    n_e, n_n = mesh.n_e, mesh.n_n
+    g = torch.Generator(device="cuda").manual_seed(cells * 100 + nq)
+    DS = torch.randn((n_e * nq, 6, 6), dtype=torch.float64, device="cuda", generator=g) * 1e4
+    K = dm.new_block_values()
+    dm.assemble(DS, K)
+    d = [torch.from_numpy(x).cuda().view(n_e, nq, 10) for x in dphi]
+    B = torch.zeros((n_e, nq, 6, 10, 3), dtype=torch.float64, device="cuda")
+    for c in range(3):
+        B[:, :, c, :, c] = d[c]
+    for row, (i, j) in ((3, (0, 1)), (4, (1, 2)), (5, (0, 2))):
+        B[:, :, row, :, i], B[:, :, row, :, j] = d[j], d[i]
+    B = B.reshape(n_e, nq, 6, 30)
+    D = 0.5 * (DS + DS.transpose(1, 2)).view(n_e, nq, 6, 6)
+    Ke = torch.einsum("eq,eqsl,eqst,eqtm->elm", torch.from_numpy(w).cuda().view(n_e, nq), B, D, B)
+    elem = torch.from_numpy(mesh.elem.T.astype(np.int64)).cuda()
+    a, b = torch.broadcast_tensors(elem[:, :, None], elem[:, None, :])
+    _, slot = torch.unique((a * n_n + b).reshape(-1), return_inverse=True)
+    ref = torch.zeros((dm.n_blocks, 9), dtype=torch.float64, device="cuda")
+    ref.index_add_(0, slot, Ke.view(n_e, 10, 3, 10, 3).transpose(2, 3).reshape(-1, 9))
+    assert (K.view(-1, 9) - ref).abs().max() <= 1e-12 * ref.abs().max()
