@@ -64,7 +64,6 @@ struct sg_krylov {
     // (GR_CTAS x 64 x 64) and the kept count on the device
     double *gram = nullptr, *gpart = nullptr;
     int32_t *gkout = nullptr;
-    double *spy = nullptr;      // n x 16: interleaved products of the long-vector SpMM
     int aorth_mode = 1;
 };
 
@@ -436,7 +435,7 @@ extern "C" int sg_krylov_destroy(sg_krylov *ws) {
     cudaFree(ws->sig);
     graph_release(ws);
     cudaFree(ws->atb); cudaFree(ws->cblk); cudaFree(ws->tspart);
-    cudaFree(ws->gram); cudaFree(ws->gpart); cudaFree(ws->gkout); cudaFree(ws->spy);
+    cudaFree(ws->gram); cudaFree(ws->gpart); cudaFree(ws->gkout);
     cudaFree(ws->u); cudaFree(ws->dstate); cudaFree(ws->dscal); cudaFree(ws->dH); cudaFree(ws->dcs);
     cudaFree(ws->dsn); cudaFree(ws->dg); cudaFree(ws->dy); cudaFree(ws->dhist); cudaFree(ws->dptr);
     if (ws->cap) cudaStreamDestroy(ws->cap);
@@ -611,15 +610,14 @@ extern "C" int sg_a_orthogonalize(sg_krylov *ws, const sg_bsr *A, const double *
     // A times every input column up front (processing order i takes column k - 1 - i): the
     // products do not depend on the orthogonalisation, and one SpMM reads A once per eight
     // columns where a SpMV per column reads it k times
-    if (A->b == 3 && k >= 4 && (double)n * 8 * 8 > 48e6) {
-        // long vectors: interleaved copies of 16 columns (scratch: the block buffer and spy)
+    if (A->b == 3 && k >= 4) {
+        // interleaved copies of 16 columns (scratch: the block buffer)
         if (!ws->atb) {
             SG_CUDA(device_alloc(&ws->atb, sizeof(double) * n * 16));
             SG_CUDA(device_alloc(&ws->cblk, sizeof(double) * 256 * 16));
             SG_CUDA(device_alloc(&ws->tspart, sizeof(double) * TS_PART_CTAS * 256 * 16));
         }
-        if (!ws->spy) SG_CUDA(device_alloc(&ws->spy, sizeof(double) * n * 16));
-        rc = bsr_spmm_interleaved(*A, Avals, W + (int64_t)(k - 1) * n, -n, AWo, n, k, ws->atb, ws->spy, st);
+        rc = bsr_spmm_interleaved(*A, Avals, W + (int64_t)(k - 1) * n, -n, AWo, n, k, ws->atb, st);
     } else if (A->b == 3) {
         rc = bsr_spmm(*A, Avals, W + (int64_t)(k - 1) * n, -n, AWo, n, k, st);
     } else {
@@ -638,12 +636,18 @@ extern "C" int sg_a_orthogonalize(sg_krylov *ws, const sg_bsr *A, const double *
         const double *S = W + (int64_t)(k - 1) * n;   // processing order: column i is W's k - 1 - i
         if ((rc = gram_upper(n, k, S, -n, AWo, n, G, ws->gpart, st))) return rc;
         if ((rc = gram_recurrence(k, G, Tp, eps_add, Ta, nt, sig, ws->gkout, pmap, st))) return rc;
-        if ((rc = ts_apply(n, k, ws->gkout, pmap, S, -n, Ta, Wo, n, st))) return rc;
-        if (AW && (rc = ts_apply(n, k, ws->gkout, pmap, AWo, n, Ta, AW, n, st))) return rc;
+        const bool in_place = k <= TS_DIRECT_MAX;   // U straight into W
+        if (in_place) {
+            rc = ts_apply_pair(n, k, ws->gkout, pmap, S, -n, W, n, AWo, n, AW, n, Ta, st);
+        } else {
+            rc = ts_apply(n, k, ws->gkout, pmap, S, -n, Ta, Wo, n, st);
+            if (!rc && AW) rc = ts_apply(n, k, ws->gkout, pmap, AWo, n, Ta, AW, n, st);
+        }
+        if (rc) return rc;
         int32_t ko = 0;
         SG_CUDA(cudaMemcpyAsync(&ko, ws->gkout, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         SG_CUDA(cudaStreamSynchronize(st));
-        if (ko > 0)
+        if (ko > 0 && !in_place)
             SG_CUDA(cudaMemcpyAsync(W, Wo, sizeof(double) * n * ko, cudaMemcpyDeviceToDevice, st));
         *k_out = ko;
         SG_CUDA(cudaStreamSynchronize(st));

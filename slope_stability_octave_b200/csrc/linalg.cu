@@ -333,15 +333,52 @@ static void spmm_pass(const sg_bsr &A, int G, const double *vals, const double *
     }
 }
 
+// Column-major -> node-interleaved copy of KC columns (node j's three components of all KC columns
+// are one run of 3 KC doubles, [component][column]) through shared-memory tiles of 64 rows:
+// both sides are coalesced.
+constexpr int PK_ROWS = 64;
+template <int KC>
+__global__ void __launch_bounds__(256) k_pack_tiles(int64_t n, int kc, const double *__restrict__ X, int64_t ldx,
+                                                    double *__restrict__ Xi) {
+    __shared__ double t[PK_ROWS][KC + 1];
+    const int64_t ntiles = (n + PK_ROWS - 1) / PK_ROWS;
+    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int64_t r0 = tile * PK_ROWS;
+        __syncthreads();
+        for (int e = threadIdx.x; e < PK_ROWS * KC; e += blockDim.x) {
+            const int c = e / PK_ROWS, r = e - c * PK_ROWS;
+            const int64_t rr = r0 + r;
+            t[r][c] = (c < kc && rr < n) ? X[(int64_t)c * ldx + rr] : 0.0;
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < PK_ROWS * KC; e += blockDim.x) {
+            const int r = e / KC, c = e - r * KC;
+            const int64_t rr = r0 + r;
+            if (rr < n) Xi[rr * KC + c] = t[r][c];
+        }
+    }
+}
 // Node-interleaved SpMM for many vectors: the KC (8 or 16) columns of a pass are packed so that
 // node j's three components of all KC columns are one contiguous run of 3 KC doubles
 // ([component][column]); a block's x gather is then 24 KC contiguous bytes however far apart
 // the original columns lie.  A warp computes one block row (the lane mapping is described at
 // the kernel); the sums are combined in a fixed order, so the result is reproducible.
+// The results of a CTA's rows, staged column by column in shared memory, into Y's columns.
+constexpr int SM_ROWS = 64, SM_LD = SM_ROWS * 3 + 1;
+__device__ __forceinline__ void spmm_columns_out(const double *sY, int nr, int64_t r0, int kc, double *__restrict__ Y,
+                                                 int64_t ldy) {
+    for (int e = threadIdx.x; e < kc * nr; e += blockDim.x) {
+        const int c = e / nr, r = e - c * nr;
+        Y[c * ldy + r0 + r] = sY[c * SM_LD + r];
+    }
+}
+
 template <int KC>
 __global__ void __launch_bounds__(256) k_spmm3i(int64_t nrows, int64_t rows_per_cta, const int32_t *__restrict__ rp,
                                                 const int32_t *__restrict__ col, const double *__restrict__ vals,
-                                                const double *__restrict__ Xi, double *__restrict__ Yi) {
+                                                const double *__restrict__ Xi, int kc, double *__restrict__ Y,
+                                                int64_t ldy) {
+    __shared__ double sY[KC][SM_LD];
     // a warp per block row; lane = (block slot bs in 0 .. 32/KC - 1, column c in 0 .. KC - 1):
     // the warp takes the row's blocks 32/KC at a time, the lanes of a slot load their block's
     // nine values together (coalesced requests) and hand them round by shuffles, each lane
@@ -386,59 +423,14 @@ __global__ void __launch_bounds__(256) k_spmm3i(int64_t nrows, int64_t rows_per_
             y2 += __shfl_xor_sync(0xffffffffu, y2, off);
         }
         if (bs == 0) {
-            double *yr = Yi + row * 3 * KC + c;
-            yr[0] = y0;
-            yr[KC] = y1;
-            yr[2 * KC] = y2;
+            const int r = (int)(row - r0) * 3;
+            sY[c][r] = y0;
+            sY[c][r + 1] = y1;
+            sY[c][r + 2] = y2;
         }
     }
-}
-
-// Column-major <-> node-interleaved copies through shared-memory tiles of 64 rows x KC
-// columns: every global access runs along a column (read) or along the interleaved rows
-// (write) of the tile, so both sides are coalesced.
-constexpr int PK_ROWS = 64;
-template <int KC>
-__global__ void __launch_bounds__(256) k_pack_tiles(int64_t n, int kc, const double *__restrict__ X, int64_t ldx,
-                                                    double *__restrict__ Xi) {
-    __shared__ double t[PK_ROWS][KC + 1];
-    const int64_t ntiles = (n + PK_ROWS - 1) / PK_ROWS;
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int64_t r0 = tile * PK_ROWS;
-        __syncthreads();
-        for (int e = threadIdx.x; e < PK_ROWS * KC; e += blockDim.x) {
-            const int c = e / PK_ROWS, r = e - c * PK_ROWS;
-            const int64_t rr = r0 + r;
-            t[r][c] = (c < kc && rr < n) ? X[(int64_t)c * ldx + rr] : 0.0;
-        }
-        __syncthreads();
-        for (int e = threadIdx.x; e < PK_ROWS * KC; e += blockDim.x) {
-            const int r = e / KC, c = e - r * KC;
-            const int64_t rr = r0 + r;
-            if (rr < n) Xi[rr * KC + c] = t[r][c];
-        }
-    }
-}
-template <int KC>
-__global__ void __launch_bounds__(256) k_unpack_tiles(int64_t n, int kc, const double *__restrict__ Yi,
-                                                      double *__restrict__ Y, int64_t ldy) {
-    __shared__ double t[PK_ROWS][KC + 1];
-    const int64_t ntiles = (n + PK_ROWS - 1) / PK_ROWS;
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int64_t r0 = tile * PK_ROWS;
-        __syncthreads();
-        for (int e = threadIdx.x; e < PK_ROWS * KC; e += blockDim.x) {
-            const int r = e / KC, c = e - r * KC;
-            const int64_t rr = r0 + r;
-            t[r][c] = rr < n ? Yi[rr * KC + c] : 0.0;
-        }
-        __syncthreads();
-        for (int e = threadIdx.x; e < PK_ROWS * KC; e += blockDim.x) {
-            const int c = e / PK_ROWS, r = e - c * PK_ROWS;
-            const int64_t rr = r0 + r;
-            if (c < kc && rr < n) Y[(int64_t)c * ldy + rr] = t[r][c];
-        }
-    }
+    __syncthreads();
+    spmm_columns_out(&sY[0][0], (int)(rend - r0) * 3, r0 * 3, kc, Y, ldy);
 }
 
 // k_spmm3i for 16 columns with a column pair per lane: lane = (block slot bs in 0..3,
@@ -449,11 +441,19 @@ __global__ void __launch_bounds__(256) k_unpack_tiles(int64_t n, int kc, const d
 // Each step issues the loads of two groups of four blocks before either group's products
 // (eight x gathers in flight per warp), and a CTA owns rows_per_cta consecutive rows that its
 // warps walk in order, so the x runs of neighbouring rows are reused from L1.
+// What bounds it: the L1 data pipe (gathers of 384 bytes a block, and two 32-bit shuffles per
+// value).  Measured on B200, 16 columns: 28.3M blocks 1.63 ms with the results written column by
+// column (1.57 + 0.13 ms with an interleaved result and an unpacking pass), 6.1M blocks 0.39 ms where
+// column-wise gathers of 8 columns took 0.52.  Tried against it: the products as FP64 MMAs with the
+// block row as three of eight tile rows, values straight into the fragments (2.0-2.4 ms: fewer
+// instructions, but twice the requests for the values), rows in bricks of 2 to 8 nodes a side
+// (1.67-2.0 ms: the gathers already hit L2, and its rate is not the bound).
 __global__ void __launch_bounds__(256, 4) k_spmm3p(int64_t nrows, int64_t rows_per_cta,
                                                 const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
-                                                const double *__restrict__ vals, const double *__restrict__ Xi,
-                                                double *__restrict__ Yi) {
+                                                const double *__restrict__ vals, const double *__restrict__ Xi, int kc,
+                                                double *__restrict__ Y, int64_t ldy) {
     constexpr int KC = 16, NS = 4, UNR = 2;
+    __shared__ double sY[KC][SM_LD];
     const int lane = threadIdx.x & 31, s = lane & 7, bs = lane >> 3, base = lane & ~7;
     const int64_t r0 = (int64_t)blockIdx.x * rows_per_cta;
     const int64_t rend = r0 + rows_per_cta < nrows ? r0 + rows_per_cta : nrows;
@@ -509,20 +509,22 @@ __global__ void __launch_bounds__(256, 4) k_spmm3p(int64_t nrows, int64_t rows_p
                 y[r][1] += __shfl_xor_sync(0xffffffffu, y[r][1], off);
             }
         if (bs == 0) {
-            double2 *yr = reinterpret_cast<double2 *>(Yi + row * 3 * KC) + s;
 #pragma unroll
-            for (int r = 0; r < 3; ++r) yr[r * KC / 2] = make_double2(y[r][0], y[r][1]);
+            for (int r = 0; r < 3; ++r) {
+                sY[2 * s][(int)(row - r0) * 3 + r] = y[r][0];
+                sY[2 * s + 1][(int)(row - r0) * 3 + r] = y[r][1];
+            }
         }
     }
+    __syncthreads();
+    spmm_columns_out(&sY[0][0], (int)(rend - r0) * 3, r0 * 3, kc, Y, ldy);
 }
 
 int bsr_spmm_interleaved(const sg_bsr &A, const double *vals, const double *X, int64_t ldx, double *Y, int64_t ldy,
-                         int k, double *Xi, double *Yi, cudaStream_t st) {
+                         int k, double *Xi, cudaStream_t st) {
     if (A.b != 3) return set_error(SG_ERR_ARG, "bsr_spmm: 3x3 blocks only");
     const int64_t n = A.n_rows * 3;
-    // 16 columns per pass with a column pair per lane (k_spmm3p, about 10 % less per column
-    // than the 8-column k_spmm3i at 32-64 columns); a last pass of at most 8 columns takes
-    // k_spmm3i, which reads half the gathered bytes of a half-empty 16-column pass
+    // 16 columns per pass; a last pass of at most 8 columns takes half the gathered bytes and MMAs
     for (int c0 = 0; c0 < k;) {
         const int rest = k - c0;
         const int KC = rest > 8 ? 16 : 8;
@@ -531,15 +533,14 @@ int bsr_spmm_interleaved(const sg_bsr &A, const double *vals, const double *X, i
         instr_units(IK_SPMM_AORTH, kc);
         const int64_t tiles = (n + PK_ROWS - 1) / PK_ROWS;
         const unsigned gt = grid_for(tiles * 256, 256, 8);
-        const int64_t rpc = chunk_len(A.n_rows, 8, 64);
+        const int64_t rpc = chunk_len(A.n_rows, 8, SM_ROWS);
+        const unsigned gr = grid_chunks(A.n_rows, rpc);
         if (KC == 16) {
             k_pack_tiles<16><<<gt, 256, 0, st>>>(n, kc, X + c0 * ldx, ldx, Xi);
-            k_spmm3p<<<grid_chunks(A.n_rows, rpc), 256, 0, st>>>(A.n_rows, rpc, A.d_row_ptr, A.d_col, vals, Xi, Yi);
-            k_unpack_tiles<16><<<gt, 256, 0, st>>>(n, kc, Yi, Y + c0 * ldy, ldy);
+            k_spmm3p<<<gr, 256, 0, st>>>(A.n_rows, rpc, A.d_row_ptr, A.d_col, vals, Xi, kc, Y + c0 * ldy, ldy);
         } else {
             k_pack_tiles<8><<<gt, 256, 0, st>>>(n, kc, X + c0 * ldx, ldx, Xi);
-            k_spmm3i<8><<<grid_chunks(A.n_rows, rpc), 256, 0, st>>>(A.n_rows, rpc, A.d_row_ptr, A.d_col, vals, Xi, Yi);
-            k_unpack_tiles<8><<<gt, 256, 0, st>>>(n, kc, Yi, Y + c0 * ldy, ldy);
+            k_spmm3i<8><<<gr, 256, 0, st>>>(A.n_rows, rpc, A.d_row_ptr, A.d_col, vals, Xi, kc, Y + c0 * ldy, ldy);
         }
         instr_end(tk, st);
         SG_CUDA(cudaGetLastError());
@@ -893,71 +894,11 @@ __device__ __forceinline__ void dmma(double &c0, double &c1, double a, double b)
                  : "d"(a), "d"(b));
 }
 
-// Partial sums of one 16 NA x 16 NA tile of G (rows m0 + [0, 16 NA), columns i0 + [0, 16 NA))
-// over this CTA's row range, in tiles of GR_R rows staged in shared memory ([column][row],
-// padded) by 8-byte cp.async, two stages; thread (mb, ib) owns the entries
-// (m0 + mb + 16 a, i0 + ib + 16 b).  part: gridDim.x x (16 NA)^2.  On a diagonal tile
-// (DIAG, m0 == i0) the products with a > b, all below the diagonal, are not formed.
-constexpr int GR_R = 32, GR_LD = GR_R + 1;
-template <int NA, bool DIAG>
-__global__ void __launch_bounds__(256) k_gram_partial(int64_t n, int k, const double *__restrict__ S, int64_t lds,
-                                                      const double *__restrict__ AS, int64_t ldas, int m0, int i0,
-                                                      double *__restrict__ part) {
-    constexpr int TW = 16 * NA;
-    extern __shared__ double gsm[];   // [2 stages][S tile, AS tile][TW][GR_LD]
-    const int t = threadIdx.x, ib = t & 15, mb = t >> 4;
-    const int64_t chunk = ((n + gridDim.x - 1) / gridDim.x + GR_R - 1) / GR_R * GR_R;
-    const int64_t r0 = blockIdx.x * chunk, r1 = min(n, r0 + chunk);
-    double acc[NA][NA];
-#pragma unroll
-    for (int a = 0; a < NA; ++a)
-#pragma unroll
-        for (int b = 0; b < NA; ++b) acc[a][b] = 0.0;
-    auto stage = [&](int st, int64_t rt) {
-        double *sS = gsm + st * 2 * TW * GR_LD, *sA = sS + TW * GR_LD;
-        for (int e = t; e < TW * GR_R; e += 256) {
-            const int c = e / GR_R, r = e - c * GR_R;
-            const int64_t row = rt + r;
-            const int cm = m0 + c, ci = i0 + c;
-            if (row < r1 && cm < k) cp_async8(sS + c * GR_LD + r, S + cm * lds + row);
-            else sS[c * GR_LD + r] = 0.0;
-            if (row < r1 && ci < k) cp_async8(sA + c * GR_LD + r, AS + ci * ldas + row);
-            else sA[c * GR_LD + r] = 0.0;
-        }
-    };
-    if (r0 < r1) stage(0, r0);
-    cp_async_commit();
-    int it = 0;
-    for (int64_t rt = r0; rt < r1; rt += GR_R, ++it) {
-        if (rt + GR_R < r1) stage((it + 1) & 1, rt + GR_R);
-        cp_async_commit();
-        cp_async_wait1();
-        __syncthreads();
-        const double *sS = gsm + (it & 1) * 2 * TW * GR_LD, *sA = sS + TW * GR_LD;
-#pragma unroll 4
-        for (int r = 0; r < GR_R; ++r) {
-            double sv[NA], xv[NA];
-#pragma unroll
-            for (int a = 0; a < NA; ++a) sv[a] = sS[(mb + 16 * a) * GR_LD + r];
-#pragma unroll
-            for (int b = 0; b < NA; ++b) xv[b] = sA[(ib + 16 * b) * GR_LD + r];
-#pragma unroll
-            for (int a = 0; a < NA; ++a)
-#pragma unroll
-                for (int b = 0; b < NA; ++b)
-                    if (!DIAG || a <= b) acc[a][b] += sv[a] * xv[b];   // (a > b): m > i, unused
-        }
-        __syncthreads();
-    }
-    double *out = part + (int64_t)blockIdx.x * TW * TW;
-#pragma unroll
-    for (int a = 0; a < NA; ++a)
-#pragma unroll
-        for (int b = 0; b < NA; ++b) out[(mb + 16 * a) * TW + ib + 16 * b] = acc[a][b];
-}
-
-// k_gram_partial for 64 x 64 tiles on the FP64 tensor cores (mma.sync m8n8k4 .f64): the
-// same row tiles and stages (pitch padded to GR_R + 4 for conflict-free fragment reads);
+constexpr int GR_R = 32;   // rows per stage of the 64 x 64 Gram tiles
+// Partial sums of one 64 x 64 tile of G (rows m0 + [0, 64), columns i0 + [0, 64)) over this CTA's
+// row range, for more than 48 columns, on the FP64 tensor cores (mma.sync m8n8k4 .f64): row tiles
+// of GR_R rows staged in shared memory by 8-byte cp.async, two stages ([column][row], pitch padded
+// to GR_R + 4 for conflict-free fragment reads);
 // warp w owns G rows m0 + 32 (w & 1) .. + 32 and columns i0 + 16 (w >> 1) .. + 16 as 4 x 2
 // tiles of 8 x 8; A = S' (a = S[row t][column m0 + g]), B = AS (b = AS[row t][column g]).
 constexpr int GM_TW = 64, GM_LD = GR_R + 4;
@@ -1020,6 +961,99 @@ __global__ void __launch_bounds__(256) k_gram_partial_mma(int64_t n, int k, cons
             for (int h = 0; h < 2; ++h) out[(wm + 8 * i + g) * GM_TW + wi + 8 * j + 2 * t + h] = acc[i][j][h];
 }
 
+// The Gram matrix of up to 8 NB <= 48 columns in one pass over S and A S on the FP64 tensor cores:
+// stages of GD_R rows of all columns in shared memory ([column][row], pitch GD_R + 4: no bank conflict in
+// the fragment reads), three in flight by 8-byte cp.async; warp w takes the row quads w, w + 4, ...
+// of a stage and accumulates every tile on or above the diagonal, and a CTA adds its warps' sums in
+// warp order, so each column is read once.  part: gridDim.x x (8 NB)^2, tiles below the diagonal unset.
+//
+// What bounds it: the two reads (16 bytes per row and column).  The tiles this replaces gave each
+// thread one product per two shared reads: 1.04-1.06 ms for 15 and 38 columns of 3.0M rows;
+// fragments straight from global memory (32-byte runs) 0.65 and 1.42 ms, this 0.51 for 38 columns.
+constexpr int GD_THREADS = 128, GD_WARPS = GD_THREADS / 32, GD_R = 32, GD_LD = GD_R + 4, GD_STAGES = 3;
+template <int NB>
+__global__ void __launch_bounds__(GD_THREADS) k_gram_direct(int64_t n, int k, const double *__restrict__ S, int64_t lds,
+                                                            const double *__restrict__ AS, int64_t ldas,
+                                                            double *__restrict__ part) {
+    constexpr int NT = NB * (NB + 1) / 2, COLS = 8 * NB;
+    extern __shared__ double gsm[];   // [stage][S, AS][COLS][GD_LD]; afterwards the warps' sums
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int64_t chunk = ((n + gridDim.x - 1) / gridDim.x + GD_R - 1) / GD_R * GD_R;
+    const int64_t r0 = blockIdx.x * chunk, r1 = r0 + chunk < n ? r0 + chunk : n;
+    double acc[NT][2];
+#pragma unroll
+    for (int p = 0; p < NT; ++p) acc[p][0] = acc[p][1] = 0.0;
+    auto stage = [&](int st, int64_t rt) {
+        double *d = gsm + st * 2 * COLS * GD_LD;
+        for (int e = threadIdx.x; e < 2 * COLS * GD_R; e += GD_THREADS) {
+            const int cc = e / GD_R, r = e - cc * GD_R, c = cc < COLS ? cc : cc - COLS;
+            const int64_t row = rt + r;
+            if (row < r1 && c < k) cp_async8(d + cc * GD_LD + r, (cc < COLS ? S + c * lds : AS + c * ldas) + row);
+            else d[cc * GD_LD + r] = 0.0;
+        }
+    };
+#pragma unroll
+    for (int s = 0; s < GD_STAGES - 1; ++s) {
+        if (r0 + s * GD_R < r1) stage(s, r0 + s * GD_R);
+        cp_async_commit();
+    }
+    int it = 0;
+    for (int64_t rt = r0; rt < r1; rt += GD_R, ++it) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(GD_STAGES - 2) : "memory");
+        __syncthreads();
+        const int64_t rn = rt + (GD_STAGES - 1) * GD_R;
+        if (rn < r1) stage((it + GD_STAGES - 1) % GD_STAGES, rn);
+        cp_async_commit();
+        const double *sS = gsm + (it % GD_STAGES) * 2 * COLS * GD_LD, *sA = sS + COLS * GD_LD;
+#pragma unroll
+        for (int h = 0; h < GD_R / 4 / GD_WARPS; ++h) {
+            const int r = 4 * (warp + GD_WARPS * h) + t;
+            double a[NB], b[NB];
+#pragma unroll
+            for (int i = 0; i < NB; ++i) {
+                a[i] = sS[(8 * i + g) * GD_LD + r];
+                b[i] = sA[(8 * i + g) * GD_LD + r];
+            }
+#pragma unroll
+            for (int i = 0, p = 0; i < NB; ++i)
+#pragma unroll
+                for (int j = i; j < NB; ++j, ++p) dmma(acc[p][0], acc[p][1], a[i], b[j]);
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < NT; ++p) {
+        gsm[(warp * NT + p) * 64 + g * 8 + 2 * t] = acc[p][0];
+        gsm[(warp * NT + p) * 64 + g * 8 + 2 * t + 1] = acc[p][1];
+    }
+    __syncthreads();
+    double *out = part + (int64_t)blockIdx.x * COLS * COLS;
+    for (int e = threadIdx.x; e < NT * 64; e += GD_THREADS) {
+        double v = 0.0;
+#pragma unroll
+        for (int q = 0; q < GD_WARPS; ++q) v += gsm[q * NT * 64 + e];
+        int p = e >> 6, i = 0;
+        while (p >= NB - i) p -= NB - i++;
+        out[(8 * i + ((e >> 3) & 7)) * COLS + 8 * (i + p) + (e & 7)] = v;
+    }
+}
+
+template <int NB>
+static int gram_direct(int64_t n, int k, const double *S, int64_t lds, const double *AS, int64_t ldas, double *part,
+                       cudaStream_t st) {
+    constexpr int stages = GD_STAGES * 2 * 8 * NB * GD_LD, sums = GD_WARPS * NB * (NB + 1) / 2 * 64;
+    constexpr size_t smem = sizeof(double) * (stages > sums ? stages : sums);
+    static thread_local bool configured = false;
+    if (!configured) {
+        SG_CUDA(cudaFuncSetAttribute(k_gram_direct<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        configured = true;
+    }
+    k_gram_direct<NB><<<GR_CTAS, GD_THREADS, smem, st>>>(n, k, S, lds, AS, ldas, part);
+    SG_CUDA(cudaGetLastError());
+    return SG_OK;
+}
+
 // G(m0 + ml, i0 + il) = the sum of the CTAs' partials: a warp per entry, lane l adding the
 // partials l, l + 32, ... and a fixed shuffle tree combining the lanes (ldg: G's leading
 // dimension)
@@ -1029,7 +1063,7 @@ __global__ void k_gram_reduce(int k, int TW, int nparts, const double *__restric
     const int nw = (gridDim.x * blockDim.x) >> 5;
     for (int o = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; o < TW * TW; o += nw) {
         const int ml = o / TW, il = o - ml * TW;
-        if (m0 + ml >= k || i0 + il >= k) continue;   // uniform over the warp
+        if (m0 + ml >= k || i0 + il >= k || m0 + ml > i0 + il) continue;   // uniform over the warp
         double s = 0.0;
         for (int p = lane; p < nparts; p += 32) s += part[(int64_t)p * TW * TW + o];
 #pragma unroll
@@ -1119,127 +1153,40 @@ __global__ void __launch_bounds__(256) k_gram_recurrence(int k, const double *__
     }
 }
 
-// Y(:, o) = X(:, 0:k) Ta(:, o) for o < *kout, output columns in chunks of 8 NJ (blockIdx.y):
-// X rows in tiles of TA_R, columns of X (and rows of Ta) in stages of TA_MC through shared
-// memory (8-byte cp.async, two stages); thread (lane, warp) owns rows lane + 32 q and output
-// columns o0 + warp NJ + j.
-constexpr int TA_R = 128, TA_MC = 16;
-template <int NJ>
-__global__ void __launch_bounds__(256, (NJ > 4 ? 2 : 3)) k_ts_apply(int64_t n, int k, const int32_t *__restrict__ kout,
-                                                  const int32_t *__restrict__ pmap, const double *__restrict__ X,
-                                                  int64_t ldx, const double *__restrict__ Ta, double *__restrict__ Y,
-                                                  int64_t ldy) {
-    constexpr int OC = 8 * NJ;
-    __shared__ double sX[2][TA_MC][TA_R];
-    __shared__ __align__(16) double sT[2][TA_MC][OC];
-    const int ko = *kout;
-    const int o0 = blockIdx.y * OC;
-    if (o0 >= ko) return;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // the chunk's columns depend on inputs 0 .. pmap[o0] only (Ta is zero below)
-    const int kk = min(k, pmap[o0] + 1);
-    const int nmc = (kk + TA_MC - 1) / TA_MC;
-    const int64_t ntiles = (n + TA_R - 1) / TA_R;
-    const int64_t nsteps = ((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x) * nmc;   // (tile, chunk) pairs
-    if (blockIdx.x >= ntiles) return;
-    auto stage = [&](int st, int64_t s) {
-        const int64_t rt = (blockIdx.x + (s / nmc) * gridDim.x) * TA_R;
-        const int mc = (int)(s % nmc) * TA_MC;
-        for (int e = tid; e < TA_MC * TA_R; e += 256) {
-            const int cc = e / TA_R, r = e - cc * TA_R;
-            const int64_t row = rt + r;
-            const int col = mc + cc;
-            if (row < n && col < kk) cp_async8(&sX[st][cc][r], X + col * ldx + row);
-            else sX[st][cc][r] = 0.0;
-        }
-        for (int e = tid; e < TA_MC * OC; e += 256) {
-            const int cc = e / OC, oo = e - cc * OC;
-            const int m = mc + cc, o = o0 + oo;
-            sT[st][cc][oo] = (m < kk && o < ko) ? Ta[(int64_t)m * k + o] : 0.0;
-        }
-    };
-    double acc[4][NJ];
-    stage(0, 0);
-    cp_async_commit();
-    for (int64_t s = 0; s < nsteps; ++s) {
-        if (s % nmc == 0) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-#pragma unroll
-                for (int j = 0; j < NJ; ++j) acc[q][j] = 0.0;
-        }
-        if (s + 1 < nsteps) stage((int)((s + 1) & 1), s + 1);
-        cp_async_commit();
-        cp_async_wait1();
-        __syncthreads();
-        const int st = (int)(s & 1);
-#pragma unroll 4
-        for (int cc = 0; cc < TA_MC; ++cc) {
-            double xv[4], tw[NJ];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) xv[q] = sX[st][cc][lane + 32 * q];
-            if constexpr (NJ % 2 == 0) {   // the warp's NJ coefficients as NJ/2 16-byte broadcasts
-                const double2 *t2 = reinterpret_cast<const double2 *>(&sT[st][cc][warp * NJ]);
-#pragma unroll
-                for (int j = 0; j < NJ / 2; ++j) {
-                    const double2 v = t2[j];
-                    tw[2 * j] = v.x;
-                    tw[2 * j + 1] = v.y;
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < NJ; ++j) tw[j] = sT[st][cc][warp * NJ + j];
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-#pragma unroll
-                for (int j = 0; j < NJ; ++j) acc[q][j] += xv[q] * tw[j];
-        }
-        __syncthreads();
-        if (s % nmc == nmc - 1) {
-            const int64_t rt = (blockIdx.x + (s / nmc) * gridDim.x) * TA_R;
-#pragma unroll
-            for (int j = 0; j < NJ; ++j) {
-                const int o = o0 + warp * NJ + j;
-                if (o >= ko) continue;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int64_t row = rt + lane + 32 * q;
-                    if (row < n) Y[o * ldy + row] = acc[q][j];
-                }
-            }
-        }
-    }
-}
+constexpr int TA_R = 128;   // rows per tile of the products beyond 48 columns
 
 int gram_upper(int64_t n, int k, const double *S, int64_t lds, const double *AS, int64_t ldas, double *G,
                double *part, cudaStream_t st) {
     if (k <= 0) return SG_OK;
-    const int NA = k <= 16 ? 1 : (k <= 32 ? 2 : (k <= 48 ? 3 : 4));
-    const int TW = 16 * NA;
-    const size_t smem = sizeof(double) * 2 * 2 * TW * GR_LD;
+    if (k <= 48) {   // one pass, every tile in registers (84 accumulator registers at 48 columns)
+        count_launch(2);
+        const int NB = (k + 7) / 8, TW = 8 * NB;
+        int rc = SG_OK;
+        switch (NB) {
+            case 1: rc = gram_direct<1>(n, k, S, lds, AS, ldas, part, st); break;
+            case 2: rc = gram_direct<2>(n, k, S, lds, AS, ldas, part, st); break;
+            case 3: rc = gram_direct<3>(n, k, S, lds, AS, ldas, part, st); break;
+            case 4: rc = gram_direct<4>(n, k, S, lds, AS, ldas, part, st); break;
+            case 5: rc = gram_direct<5>(n, k, S, lds, AS, ldas, part, st); break;
+            default: rc = gram_direct<6>(n, k, S, lds, AS, ldas, part, st); break;
+        }
+        if (rc) return rc;
+        k_gram_reduce<<<(TW * TW * 32 + 255) / 256, 256, 0, st>>>(k, TW, GR_CTAS, part, 0, 0, G, k);
+        SG_CUDA(cudaGetLastError());
+        return SG_OK;
+    }
     static thread_local bool configured = false;
-    if (!configured) {   // stages of 48- and 64-wide tiles exceed the default 48 KB
-        SG_CUDA(cudaFuncSetAttribute(k_gram_partial<3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(sizeof(double) * 2 * 2 * 48 * GR_LD)));
+    if (!configured) {   // the stages exceed the default 48 KB
         SG_CUDA(cudaFuncSetAttribute(k_gram_partial_mma, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)GM_SMEM));
         configured = true;
     }
-    const int nt = (k + TW - 1) / TW;
+    const int TW = GM_TW, nt = (k + TW - 1) / TW;
     for (int p = 0; p < nt; ++p)
         for (int q = 0; q <= p; ++q) {
             count_launch(2);
-            const int m0 = q * TW, i0 = p * TW;
-            switch (NA) {
-                case 1: k_gram_partial<1, true><<<GR_CTAS, 256, smem, st>>>(n, k, S, lds, AS, ldas, m0, i0, part); break;
-                case 2: k_gram_partial<2, true><<<GR_CTAS, 256, smem, st>>>(n, k, S, lds, AS, ldas, m0, i0, part); break;
-                case 3: k_gram_partial<3, true><<<GR_CTAS, 256, smem, st>>>(n, k, S, lds, AS, ldas, m0, i0, part); break;
-                default:   // 64-wide tiles on the FP64 tensor cores
-                    k_gram_partial_mma<<<GR_CTAS, 256, GM_SMEM, st>>>(n, k, S, lds, AS, ldas, m0, i0, part);
-                    break;
-            }
-            k_gram_reduce<<<(TW * TW * 32 + 255) / 256, 256, 0, st>>>(k, TW, GR_CTAS, part, m0, i0, G, k);
+            k_gram_partial_mma<<<GR_CTAS, 256, GM_SMEM, st>>>(n, k, S, lds, AS, ldas, q * TW, p * TW, part);
+            k_gram_reduce<<<(TW * TW * 32 + 255) / 256, 256, 0, st>>>(k, TW, GR_CTAS, part, q * TW, p * TW, G, k);
             SG_CUDA(cudaGetLastError());
         }
     return SG_OK;
@@ -1263,8 +1210,8 @@ int gram_recurrence(int k, const double *G, double *Tp, double eps, double *Ta, 
     return SG_OK;
 }
 
-// The 64-column variant of k_ts_apply on the FP64 tensor cores (mma.sync m8n8k4 .f64, the
-// FP64 MMA of sm_100a): CTA tile 128 rows x 64 output columns, inputs in stages of TM_MC
+// Y(:, o) = X(:, 0:k) Ta(:, o) for o < *kout and more than 48 columns, on the FP64 tensor cores
+// (mma.sync m8n8k4 .f64, the FP64 MMA of sm_100a): CTA tile 128 rows x 64 output columns, inputs in stages of TM_MC
 // columns of X / rows of Ta staged by 8-byte cp.async (two stages, pitches padded by 4
 // doubles so the fragment reads are free of bank conflicts); warp w owns rows 32 (w & 3) ..
 // + 32 and columns 32 (w >> 2) .. + 32 as 4 x 4 tiles of 8 x 8, an MMA per tile and step of 4
@@ -1354,51 +1301,108 @@ __global__ void __launch_bounds__(256) k_ts_apply_mma(int64_t n, int k, const in
     }
 }
 
+// Y(:, o) = X(:, 0:k) Ta(:, o), o < *kout, for k <= 8 KB <= 48 and two pairs (X, Y) at once
+// (blockIdx.y), Ta (k x k, row-major) in shared memory.  A warp takes 8 R rows: their k inputs go
+// straight into m8n8k4 fragments (row g, input t: 64-byte runs), then each chunk of eight output
+// columns is formed from the inputs it depends on and written.  All of a row's inputs are in
+// registers before its first output is written, so Y may be X's own array in any column order.
+//
+// What bounds it: reading and writing the two bases.  38 columns of 3.0M rows: 0.79 ms for both
+// products (4.6 TB/s), against 0.88 ms each with the inputs staged in shared memory and FMAs, and
+// 0.29 ms for copying U back into place.
+template <int KB>
+__global__ void __launch_bounds__(256) k_ts_apply_direct(int64_t n, int k, const int32_t *__restrict__ kout,
+                                                         const int32_t *__restrict__ pmap, const double *X0,
+                                                         int64_t ldx0, double *Y0, int64_t ldy0, const double *X1,
+                                                         int64_t ldx1, double *Y1, int64_t ldy1,
+                                                         const double *__restrict__ Ta) {
+    constexpr int R = KB <= 3 ? 4 : 2, TP = 8 * KB + (KB % 2 ? 12 : 4);   // pitch 4 mod 16: no bank conflicts
+    __shared__ double sT[8 * KB * TP];
+    const int ko = *kout;
+    for (int e = threadIdx.x; e < 8 * KB * 8 * KB; e += blockDim.x) {
+        const int m = e / (8 * KB), o = e - m * 8 * KB;
+        sT[m * TP + o] = m < k && o < ko ? Ta[(int64_t)m * k + o] : 0.0;
+    }
+    __syncthreads();
+    const double *X = blockIdx.y ? X1 : X0;
+    double *Y = blockIdx.y ? Y1 : Y0;
+    const int64_t ldx = blockIdx.y ? ldx1 : ldx0, ldy = blockIdx.y ? ldy1 : ldy0;
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    int lim[KB];   // inputs that output chunk j depends on (decreasing in j)
+#pragma unroll
+    for (int j = 0; j < KB; ++j) lim[j] = 8 * j < ko ? pmap[8 * j] + 1 : 0;
+    const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t r0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 8 * R; r0 < n; r0 += nw * 8 * R) {
+        double a[R][2 * KB];
+#pragma unroll
+        for (int i = 0; i < 2 * KB; ++i)
+#pragma unroll
+            for (int q = 0; q < R; ++q) {
+                const int64_t row = r0 + 8 * q + g;
+                a[q][i] = row < n && 4 * i + t < k ? X[(int64_t)(4 * i + t) * ldx + row] : 0.0;
+            }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < KB; ++j) {
+            if (8 * j >= ko) break;
+            double c[R][2];
+#pragma unroll
+            for (int q = 0; q < R; ++q) c[q][0] = c[q][1] = 0.0;
+#pragma unroll
+            for (int i = 0; i < 2 * KB; ++i)
+                if (4 * i < lim[j]) {
+                    const double b = sT[(4 * i + t) * TP + 8 * j + g];
+#pragma unroll
+                    for (int q = 0; q < R; ++q) dmma(c[q][0], c[q][1], a[q][i], b);
+                }
+#pragma unroll
+            for (int q = 0; q < R; ++q) {
+                const int64_t row = r0 + 8 * q + g;
+                const int o = 8 * j + 2 * t;
+                if (row < n && o < ko) Y[(int64_t)o * ldy + row] = c[q][0];
+                if (row < n && o + 1 < ko) Y[(int64_t)(o + 1) * ldy + row] = c[q][1];
+            }
+        }
+    }
+}
+
+int ts_apply_pair(int64_t n, int k, const int32_t *kout, const int32_t *pmap, const double *X0, int64_t ldx0,
+                  double *Y0, int64_t ldy0, const double *X1, int64_t ldx1, double *Y1, int64_t ldy1, const double *Ta,
+                  cudaStream_t st) {
+    if (k <= 0 || n <= 0) return SG_OK;
+    if (k > TS_DIRECT_MAX) return set_error(SG_ERR_ARG, "ts_apply_pair: too many columns");
+    const int KB = (k + 7) / 8;
+    count_launch();
+    const dim3 grid((unsigned)std::min<int64_t>((n + 127) / 128, (int64_t)sm_count() * 8), Y1 ? 2 : 1);
+#define SG_TS(B) k_ts_apply_direct<B><<<grid, 256, 0, st>>>(n, k, kout, pmap, X0, ldx0, Y0, ldy0, X1, ldx1, Y1, ldy1, Ta)
+    switch (KB) {
+        case 1: SG_TS(1); break;
+        case 2: SG_TS(2); break;
+        case 3: SG_TS(3); break;
+        case 4: SG_TS(4); break;
+        case 5: SG_TS(5); break;
+        default: SG_TS(6); break;
+    }
+#undef SG_TS
+    SG_CUDA(cudaGetLastError());
+    return SG_OK;
+}
+
 int ts_apply(int64_t n, int k, const int32_t *kout, const int32_t *pmap, const double *X, int64_t ldx,
              const double *Ta, double *Y, int64_t ldy, cudaStream_t st) {
     if (k <= 0 || n <= 0) return SG_OK;
     const int64_t ntiles = (n + TA_R - 1) / TA_R;
-    if (k >= 64) {   // 64-column chunks on the FP64 tensor cores
-        static thread_local int resident_mma = 0;
-        if (!resident_mma) {
-            SG_CUDA(cudaFuncSetAttribute(k_ts_apply_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TM_SMEM));
-            int r = 0;
-            SG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_ts_apply_mma, 256, TM_SMEM));
-            resident_mma = std::max(1, r);
-        }
-        const dim3 grid((unsigned)std::min<int64_t>(ntiles, (int64_t)sm_count() * resident_mma),
-                        (unsigned)((k + TM_OC - 1) / TM_OC));
-        count_launch();
-        k_ts_apply_mma<<<grid, 256, TM_SMEM, st>>>(n, k, kout, pmap, X, ldx, Ta, Y, ldy);
-        SG_CUDA(cudaGetLastError());
-        return SG_OK;
-    }
-    const int nj = (k + 7) / 8;
-    const int oc = 8 * nj;
-    // CTAs resident per SM for this variant (registers and shared memory), once per variant
-    static thread_local int resident[9] = {};
-    if (!resident[nj]) {
-        const void *fn = nj == 1 ? (const void *)k_ts_apply<1> : nj == 2 ? (const void *)k_ts_apply<2>
-                       : nj == 3 ? (const void *)k_ts_apply<3> : nj == 4 ? (const void *)k_ts_apply<4>
-                       : nj == 5 ? (const void *)k_ts_apply<5> : nj == 6 ? (const void *)k_ts_apply<6>
-                       : nj == 7 ? (const void *)k_ts_apply<7> : (const void *)k_ts_apply<8>;
+    static thread_local int resident_mma = 0;
+    if (!resident_mma) {
+        SG_CUDA(cudaFuncSetAttribute(k_ts_apply_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TM_SMEM));
         int r = 0;
-        SG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, fn, 256, 0));
-        resident[nj] = std::max(1, r);
+        SG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_ts_apply_mma, 256, TM_SMEM));
+        resident_mma = std::max(1, r);
     }
-    const dim3 grid((unsigned)std::min<int64_t>(ntiles, (int64_t)sm_count() * resident[nj]),
-                    (unsigned)((k + oc - 1) / oc));
+    const dim3 grid((unsigned)std::min<int64_t>(ntiles, (int64_t)sm_count() * resident_mma),
+                    (unsigned)((k + TM_OC - 1) / TM_OC));
     count_launch();
-    switch (nj) {
-        case 1: k_ts_apply<1><<<grid, 256, 0, st>>>(n, k, kout, pmap, X, ldx, Ta, Y, ldy); break;
-        case 2: k_ts_apply<2><<<grid, 256, 0, st>>>(n, k, kout, pmap, X, ldx, Ta, Y, ldy); break;
-        case 3: k_ts_apply<3><<<grid, 256, 0, st>>>(n, k, kout, pmap, X, ldx, Ta, Y, ldy); break;
-        case 4: k_ts_apply<4><<<grid, 256, 0, st>>>(n, k, kout, pmap, X, ldx, Ta, Y, ldy); break;
-        case 5: k_ts_apply<5><<<grid, 256, 0, st>>>(n, k, kout, pmap, X, ldx, Ta, Y, ldy); break;
-        case 6: k_ts_apply<6><<<grid, 256, 0, st>>>(n, k, kout, pmap, X, ldx, Ta, Y, ldy); break;
-        case 7: k_ts_apply<7><<<grid, 256, 0, st>>>(n, k, kout, pmap, X, ldx, Ta, Y, ldy); break;
-        default: k_ts_apply<8><<<grid, 256, 0, st>>>(n, k, kout, pmap, X, ldx, Ta, Y, ldy); break;
-    }
+    k_ts_apply_mma<<<grid, 256, TM_SMEM, st>>>(n, k, kout, pmap, X, ldx, Ta, Y, ldy);
     SG_CUDA(cudaGetLastError());
     return SG_OK;
 }

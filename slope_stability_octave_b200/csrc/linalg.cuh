@@ -27,11 +27,10 @@ int rect_spmv(int br, int bc, int64_t nrows, const int32_t *rp, const int32_t *c
 int bsr_spmm(const sg_bsr &A, const double *vals, const double *X, int64_t ldx, double *Y, int64_t ldy, int k,
              cudaStream_t st);
 
-// The same product through node-interleaved copies of 16 columns at a time (Xi, Yi: 16 n
-// doubles each of scratch): for many columns of long vectors, whose column-wise gathers would
-// not stay in L2.
+// The same product through a node-interleaved copy of 16 columns at a time (Xi: 16 n doubles of
+// scratch), on the FP64 tensor cores; sums in another order than bsr_spmv's.
 int bsr_spmm_interleaved(const sg_bsr &A, const double *vals, const double *X, int64_t ldx, double *Y, int64_t ldy,
-                         int k, double *Xi, double *Yi, cudaStream_t st);
+                         int k, double *Xi, cudaStream_t st);
 
 // Reduction workspace for dot products: partial sums of `nblk` blocks per column.
 constexpr int DOT_BLOCKS = 296;  // 2 x 148 SMs
@@ -80,8 +79,14 @@ int gram_recurrence(int k, const double *G, double *Tp, double eps, double *Ta, 
                     int32_t *kout, int32_t *pmap, cudaStream_t st);
 int ts_apply(int64_t n, int k, const int32_t *kout, const int32_t *pmap, const double *X, int64_t ldx,
              const double *Ta, double *Y, int64_t ldy, cudaStream_t st);
+//   ts_apply_pair    Y0 = X0 Ta and (Y1 not null) Y1 = X1 Ta in one launch, k <= TS_DIRECT_MAX; each
+//                    Y may share its X's array
+constexpr int TS_DIRECT_MAX = 48;
+int ts_apply_pair(int64_t n, int k, const int32_t *kout, const int32_t *pmap, const double *X0, int64_t ldx0,
+                  double *Y0, int64_t ldy0, const double *X1, int64_t ldx1, double *Y1, int64_t ldy1, const double *Ta,
+                  cudaStream_t st);
 
-// Device-count variants for graph-replayed loops// Device-count variants for graph-replayed loops: m = min(cnt[0] + add, mmax) columns, basis
+// Device-count variants for graph-replayed loops: m = min(cnt[0] + add, mmax) columns, basis
 // V, or *Vp when V is null (both on the device)
 int multidot_dc(int64_t n, const int32_t *cnt, int add, int mmax, const double *V, const double *const *Vp,
                 int64_t ldv, const double *w, double *partial, double *out, cudaStream_t st);
