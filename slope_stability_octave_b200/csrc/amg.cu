@@ -71,6 +71,7 @@ struct Level {
     double *Dinv = nullptr;
     float *Dinv32 = nullptr;
     double *lmax = nullptr;        // device scalar
+    double *coef = nullptr;        // Chebyshev coefficients {c1, c2} per step
     uint8_t *d_dead = nullptr;     // per DOF: dead coarse DOF (identity row), coarse levels only
     // transfer to the next level
     std::vector<int32_t> agg;
@@ -118,8 +119,9 @@ struct sg_amg {
     int64_t nc_dense = 0;      // coarsest dense size (DOFs)
     double *Ainv = nullptr;    // dense inverse, nc_dense^2
     float *Ainv32 = nullptr;
-    double *colk = nullptr, *rowk = nullptr;   // Gauss-Jordan column block (N x NB) and row block (NB x N)
-    double *gj_pinv = nullptr;                 // inverse of the current pivot block (NB x NB)
+    double *Ainv2 = nullptr;   // second copy for its inversion (at most GJ_STEP_MAX unknowns)
+    double *colk = nullptr, *rowk = nullptr;   // beyond: Gauss-Jordan column block (N x NB), row block (NB x N)
+    double *gj_pinv = nullptr;                 // inverses of the current and the next pivot block (NB x NB each)
     double *dots = nullptr;    // reduction scratch
     // optional node-wise correction after the cycle: z += C (r - A z), C n x 3 x 3 (3D only)
     double *corrC = nullptr;
@@ -382,22 +384,32 @@ __global__ void k_dinv_apply(int64_t n, const T *__restrict__ Dinv, const T *__r
     }
 }
 
-// Chebyshev step on D^-1 A with bounds [lmax/ratio, 1.1 lmax]:
-//   first (k == 0):  d = D^-1 r / theta;               x += d
-//   next  (k >= 1):  d = c1 d + c2 D^-1 r;             x += d
-// rho_k follows rho_0 = 1/sigma, rho_{k} = 1/(2 sigma - rho_{k-1}).
-template <int B, typename T>
-__global__ void k_cheb(int64_t n, int k, double ratio, const double *__restrict__ lmax, const T *__restrict__ Dinv,
-                       const T *__restrict__ r, T *__restrict__ d, T *__restrict__ x, int x_is_zero) {
-    const double hi = 1.1 * lmax[0], lo = lmax[0] / ratio;
+// Chebyshev smoothing on D^-1 A with bounds [lmax/ratio, 1.1 lmax]: step k is
+//   d = c1 d + c2 D^-1 r (k = 0: d = c2 D^-1 r);  x += d
+// with rho_0 = 1/sigma, rho_k = 1/(2 sigma - rho_{k-1}).  The coefficients {c1, c2} of every step are
+// formed once per value update, where lambda_max is.
+__device__ __forceinline__ void cheb_coefficients(double lmax, double ratio, int deg, double *coef) {
+    const double hi = 1.1 * lmax, lo = lmax / ratio;
     const double theta = 0.5 * (hi + lo), delta = 0.5 * (hi - lo), sigma = theta / delta;
     double rho = 1.0 / sigma, c1 = 0.0, c2 = 1.0 / theta;
-    for (int s = 1; s <= k; ++s) {
-        const double rn = 1.0 / (2.0 * sigma - rho);
-        c1 = rn * rho;
-        c2 = 2.0 * rn / delta;
-        rho = rn;
+    for (int k = 0; k < deg; ++k) {
+        if (k > 0) {
+            const double rn = 1.0 / (2.0 * sigma - rho);
+            c1 = rn * rho;
+            c2 = 2.0 * rn / delta;
+            rho = rn;
+        }
+        coef[2 * k] = c1;
+        coef[2 * k + 1] = c2;
     }
+}
+
+// The vector part of a step for a given r (the others run as the epilogue of their residual,
+// cheb_step).
+template <int B, typename T>
+__global__ void k_cheb(int64_t n, int k, const double *__restrict__ coef, const T *__restrict__ Dinv,
+                       const T *__restrict__ r, T *__restrict__ d, T *__restrict__ x, int x_is_zero) {
+    const double c1 = coef[2 * k], c2 = coef[2 * k + 1];
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         T rv[B];
 #pragma unroll
@@ -742,17 +754,17 @@ static void gather_Ac_groups(int64_t nitems, int64_t pairs, const int32_t *qmap,
     }
 }
 
-// Blocks below the diagonal of a symmetric Galerkin matrix: A(dst) = A(src)'.
+// Blocks below the diagonal of a symmetric Galerkin matrix: A(dst) = A(src)'.  A thread per
+// entry, so the writes of a block are one run and its reads stay within one block (a thread per
+// block strode BC * BC values between lanes: 123 against 28 us a level on the layered slope).
 template <int BC, typename V>
 __global__ void k_mirror_blocks(int64_t n, const int32_t *__restrict__ dst, const int32_t *__restrict__ src,
                                 V *__restrict__ A) {
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
-        const V *a = A + (int64_t)src[t] * BC * BC;
-        V *o = A + (int64_t)dst[t] * BC * BC;
-#pragma unroll
-        for (int r = 0; r < BC; ++r)
-#pragma unroll
-            for (int c = 0; c < BC; ++c) o[r * BC + c] = a[c * BC + r];
+    const int64_t total = n * BC * BC;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t k = t / (BC * BC);
+        const int e = (int)(t - k * BC * BC), r = e / BC, c = e - r * BC;
+        A[(int64_t)dst[k] * BC * BC + e] = A[(int64_t)src[k] * BC * BC + c * BC + r];
     }
 }
 
@@ -775,7 +787,7 @@ static void galerkin_Ac(const Level &L, const Level &C, const V *P, const V *AP,
         gather_Ac_groups<B, BC, V>(items, L.ac_pairs, qmap, C.Aown.d_row, C.d_Acol, L.ac_plan.d_ptr, L.ac_plan.d_a,
                                    L.ac_plan.d_b, P, AP, C.d_dead, Ac, st);
     if (sym && L.n_ac_lower > 0)
-        k_mirror_blocks<BC, V><<<grid_for(L.n_ac_lower, 256), 256, 0, st>>>(L.n_ac_lower, L.d_ac_lower,
+        k_mirror_blocks<BC, V><<<grid_for(L.n_ac_lower * BC * BC, 256, 16), 256, 0, st>>>(L.n_ac_lower, L.d_ac_lower,
                                                                            L.d_ac_lower_src, Ac);
 }
 
@@ -801,51 +813,27 @@ __global__ void k_init_vec(int64_t n, double *__restrict__ v) {
 
 // lmax = sqrt(dots[0]) ; v = w / lmax
 __global__ void k_power_norm(int64_t n, const double *__restrict__ w, const double *__restrict__ dots,
-                             double *__restrict__ v, double *__restrict__ lmax) {
+                             double *__restrict__ v, double *__restrict__ lmax, double ratio, int deg,
+                             double *__restrict__ coef) {
     const double nrm = sqrt(dots[0]);
     const double inv = nrm > 0.0 ? 1.0 / nrm : 0.0;
-    if (blockIdx.x == 0 && threadIdx.x == 0) lmax[0] = nrm > 0.0 ? nrm : 1.0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        lmax[0] = nrm > 0.0 ? nrm : 1.0;
+        if (coef) cheb_coefficients(lmax[0], ratio, deg, coef);
+    }
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         v[i] = w[i] * inv;
 }
 
-// dense coarsest matrix from the block pattern
+// dense coarsest matrix (zeroed before) from the block pattern, a thread per entry
 template <int B, typename V = double>
-__global__ void k_bsr_to_dense(int64_t nrows, const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
+__global__ void k_bsr_to_dense(int64_t nblk, const int32_t *__restrict__ row_of, const int32_t *__restrict__ col,
                                const V *__restrict__ A, int64_t N, double *__restrict__ D) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nrows; i += (int64_t)gridDim.x * blockDim.x)
-        for (int32_t p = rp[i]; p < rp[i + 1]; ++p) {
-            const int64_t j = col[p];
-#pragma unroll
-            for (int a = 0; a < B; ++a)
-#pragma unroll
-                for (int b = 0; b < B; ++b) D[(i * B + a) * N + j * B + b] = A[(int64_t)p * B * B + a * B + b];
-        }
-}
-
-// Gauss-Jordan inversion (SPD, no pivoting), pivot k: save column k and the scaled row k
-__global__ void k_gj_save(int64_t N, int64_t k, const double *__restrict__ D, double *__restrict__ colk,
-                          double *__restrict__ rowk) {
-    const double piv = D[k * N + k];
-    const double ip = piv != 0.0 ? 1.0 / piv : 0.0;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < N; t += (int64_t)gridDim.x * blockDim.x) {
-        colk[t] = D[t * N + k];
-        rowk[t] = D[k * N + t] * ip;
-    }
-}
-__global__ void k_gj_update(int64_t N, int64_t k, double *__restrict__ D, const double *__restrict__ colk,
-                            const double *__restrict__ rowk) {
-    const double piv = colk[k];
-    const double ip = piv != 0.0 ? 1.0 / piv : 0.0;
-    const int64_t total = N * N;
+    const int64_t total = nblk * B * B;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = t / N, j = t - i * N;
-        double v;
-        if (i == k && j == k) v = ip;
-        else if (i == k) v = rowk[j];
-        else if (j == k) v = -colk[i] * ip;
-        else v = D[t] - colk[i] * rowk[j];
-        D[t] = v;
+        const int64_t p = t / (B * B);
+        const int e = (int)(t - p * B * B), a = e / B, b = e - a * B;
+        D[((int64_t)row_of[p] * B + a) * N + (int64_t)col[p] * B + b] = (double)A[t];
     }
 }
 
@@ -925,6 +913,98 @@ __global__ void k_gjb_update(int64_t N, int64_t k0, int nb, double *__restrict__
     }
 }
 
+// The same inversion in one launch per pivot block for matrices of at most GJ_STEP_MAX unknowns: a
+// CTA per 32 x 32 tile reads the pivot's row and column blocks from one copy of the matrix and
+// writes its tile of the other, forming its part of the scaled row block itself; the CTA of the next
+// pivot block then inverts that block in place, so the serial inversion runs beside the other
+// tiles.  Same operations in the same order as the three kernels above.
+// What bounds it: the chain tile -> pivot inverse -> next step.  On B200 350 unknowns (11 pivot
+// blocks) took 320 us in 33 launches with the kernels above and take 140 us here (12.2 us a step; the
+// pivot block inverted by one warp's shuffles, unrolled: 25 us a step).
+constexpr int64_t GJ_STEP_MAX = 2048;
+
+// In-place inverse of an nb x nb block held by a CTA of 256 threads, thread (r0, c) the entries
+// (r0 + 8 q, c): per pivot the owners publish its row and column, one barrier, everybody updates.
+__device__ __forceinline__ void gj_invert_cta(double (&v)[4], int nb, int r0, int c, double *__restrict__ Pinv) {
+    __shared__ double row[2][GJ_NB], colm[2][GJ_NB];
+    for (int k = 0; k < nb; ++k) {
+        const int b = k & 1;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (r0 + 8 * q == k) row[b][c] = v[q];
+            if (c == k) colm[b][r0 + 8 * q] = v[q];
+        }
+        __syncthreads();
+        const double piv = row[b][k];
+        const double ip = piv != 0.0 ? 1.0 / piv : 0.0;
+        const double rk = c == k ? ip : row[b][c] * ip;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int r = r0 + 8 * q;
+            v[q] = r == k ? rk : (c == k ? 0.0 : v[q]) - colm[b][r] * rk;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        if (r0 + 8 * q < nb && c < nb) Pinv[(r0 + 8 * q) * GJ_NB + c] = v[q];
+}
+
+__global__ void __launch_bounds__(256) k_gjb_first(int64_t N, int nb, const double *__restrict__ D,
+                                                   double *__restrict__ Pinv) {
+    const int c = threadIdx.x & 31, r0 = threadIdx.x >> 5;
+    double v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = r0 + 8 * q < nb && c < nb ? D[(r0 + 8 * q) * N + c] : 0.0;
+    gj_invert_cta(v, nb, r0, c, Pinv);
+}
+
+__global__ void __launch_bounds__(256) k_gjb_step(int64_t N, int K, const double *__restrict__ Din,
+                                                  double *__restrict__ Dout, const double *__restrict__ Pinv,
+                                                  double *__restrict__ Pnext) {
+    __shared__ double P[GJ_NB][GJ_NB + 1], C[GJ_NB][GJ_NB + 1], R[GJ_NB][GJ_NB + 1], Rw[GJ_NB][GJ_NB + 1];
+    const int I = blockIdx.y, J = blockIdx.x, c = threadIdx.x & 31, r0 = threadIdx.x >> 5;
+    const int64_t i0 = (int64_t)I * GJ_NB, j0 = (int64_t)J * GJ_NB, k0 = (int64_t)K * GJ_NB;
+    const int ni = (int)(N - i0 < GJ_NB ? N - i0 : GJ_NB), nj = (int)(N - j0 < GJ_NB ? N - j0 : GJ_NB);
+    const int nb = (int)(N - k0 < GJ_NB ? N - k0 : GJ_NB);
+    double d[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int r = r0 + 8 * q;
+        P[r][c] = r < nb && c < nb ? Pinv[r * GJ_NB + c] : 0.0;
+        C[r][c] = r < ni && c < nb ? Din[(i0 + r) * N + k0 + c] : 0.0;
+        R[r][c] = r < nb && c < nj ? Din[(k0 + r) * N + j0 + c] : 0.0;
+        d[q] = r < ni && c < nj ? Din[(i0 + r) * N + j0 + c] : 0.0;
+    }
+    __syncthreads();
+    if (J != K) {      // the scaled row block
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int r = r0 + 8 * q;
+            double s = 0.0;
+            for (int m = 0; m < nb; ++m) s += P[r][m] * R[m][c];
+            Rw[r][c] = s;
+        }
+        __syncthreads();
+    }
+    double v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int r = r0 + 8 * q;
+        if (I == K) {
+            v[q] = J == K ? P[r][c] : Rw[r][c];
+        } else {
+            double s = 0.0;
+            if (J == K)
+                for (int m = 0; m < nb; ++m) s += C[r][m] * P[m][c];
+            else
+                for (int m = 0; m < nb; ++m) s += C[r][m] * Rw[m][c];
+            v[q] = J == K ? -s : d[q] - s;
+        }
+        if (r < ni && c < nj) Dout[(i0 + r) * N + j0 + c] = v[q];
+    }
+    if (I == K + 1 && J == K + 1) gj_invert_cta(v, ni, r0, c, Pnext);
+}
+
 template <typename T>
 __global__ void k_dense_gemv(int64_t N, const T *__restrict__ M, const T *__restrict__ x, T *__restrict__ y) {
     // one warp per row
@@ -962,7 +1042,7 @@ __global__ void k_dense_gemv(int64_t N, const T *__restrict__ M, const T *__rest
 static int free_level(Level &l) {
     auto F = [](void *p) { if (p) cudaFree(p); };
     F(l.Aown.d_rp); F(l.Aown.d_col); F(l.d_diag_own); F(l.Aown_vals); F(l.A32); F(l.A16); F(l.Dinv); F(l.Dinv32);
-    F(l.lmax); F(l.d_dead); F(l.d_agg); F(l.T); F(l.P.d_rp); F(l.P.d_col); F(l.R.d_rp); F(l.R.d_col);
+    F(l.lmax); F(l.coef); F(l.d_dead); F(l.d_agg); F(l.T); F(l.P.d_rp); F(l.P.d_col); F(l.R.d_rp); F(l.R.d_col);
     F(l.AP.d_rp); F(l.AP.d_col); F(l.d_R_from_P); F(l.d_ac_out); F(l.d_ac_lower); F(l.d_ac_lower_src);
     F(l.Aown.d_row); F(l.P.d_row); F(l.R.d_row); F(l.AP.d_row);
     for (Plan *p : {&l.at_plan, &l.ap_plan, &l.ac_plan}) { F(p->d_ptr); F(p->d_a); F(p->d_b); }
@@ -971,10 +1051,11 @@ static int free_level(Level &l) {
     return SG_OK;
 }
 
-static int alloc_level_buffers(Level &L, int mixed) {
+static int alloc_level_buffers(Level &L, int mixed, int cheb_degree) {
     const size_t nb = (size_t)L.n * L.b;
     int rc = dalloc(&L.Dinv, nb * L.b);
     if (!rc) rc = dalloc(&L.lmax, 4);
+    if (!rc) rc = dalloc(&L.coef, 2 * (size_t)cheb_degree);
     if (!rc) rc = dalloc(&L.x, nb);
     if (!rc) rc = dalloc(&L.rhs, nb);
     if (!rc) rc = dalloc(&L.r, nb);
@@ -1143,7 +1224,8 @@ static int power_lmax(sg_amg *h, Level &L, const double *A, cudaStream_t st) {
         SG_B_DISPATCH(L.b, (k_dinv_apply<BB, double><<<grid_for(L.n, 256), 256, 0, st>>>(L.n, L.Dinv, L.t, L.r)));
         rc = multidot(nd, 1, L.r, nd, L.r, h->dots, h->dots + DOT_BLOCKS, st);
         if (rc) break;
-        k_power_norm<<<grid_for(nd, 256), 256, 0, st>>>(nd, L.r, h->dots + DOT_BLOCKS, L.pv, L.lmax);
+        k_power_norm<<<grid_for(nd, 256), 256, 0, st>>>(nd, L.r, h->dots + DOT_BLOCKS, L.pv, L.lmax, h->opt.cheb_ratio,
+                                                        h->opt.cheb_degree, it + 1 == its ? L.coef : nullptr);
     }
     SG_CUDA(cudaGetLastError());
     return rc;
@@ -1164,7 +1246,8 @@ static int power_lmax32(sg_amg *h, Level &L, cudaStream_t st) {
         SG_B_DISPATCH(L.b, (k_dinv_apply<BB, double><<<grid_for(L.n, 256), 256, 0, st>>>(L.n, L.Dinv, L.t, L.r)));
         rc = multidot(nd, 1, L.r, nd, L.r, h->dots, h->dots + DOT_BLOCKS, st);
         if (rc) break;
-        k_power_norm<<<grid_for(nd, 256), 256, 0, st>>>(nd, L.r, h->dots + DOT_BLOCKS, L.pv, L.lmax);
+        k_power_norm<<<grid_for(nd, 256), 256, 0, st>>>(nd, L.r, h->dots + DOT_BLOCKS, L.pv, L.lmax, h->opt.cheb_ratio,
+                                                        h->opt.cheb_degree, it + 1 == its ? L.coef : nullptr);
     }
     SG_CUDA(cudaGetLastError());
     return rc;
@@ -1220,22 +1303,44 @@ static int numeric_transfer(sg_amg *h, int l, cudaStream_t st) {
     return SG_OK;
 }
 
-static int numeric_coarsest(sg_amg *h, cudaStream_t st) {
+// The coarsest level's dense inverse (and its FP32 copy) from the level's values.
+template <typename V>
+static int coarsest_inverse(sg_amg *h, const V *A, cudaStream_t st) {
     Level &L = h->L.back();
-    const double *A = level_values(L);
     const int64_t N = h->nc_dense;
-    SG_CUDA(cudaMemsetAsync(h->Ainv, 0, sizeof(double) * N * N, st));
-    SG_B_DISPATCH(L.b, (k_bsr_to_dense<BB><<<grid_for(L.n, 128), 128, 0, st>>>(L.n, L.d_Arp, L.d_Acol, A, N, h->Ainv)));
-    for (int64_t k0 = 0; k0 < N; k0 += GJ_NB) {
-        const int nb = (int)std::min<int64_t>(GJ_NB, N - k0);
-        count_launch();
-        k_gjb_pivot<<<1, GJ_NB * GJ_NB, 0, st>>>(N, k0, nb, h->Ainv, h->gj_pinv);
-        k_gjb_save<<<grid_for(N * nb, 256), 256, 0, st>>>(N, k0, nb, h->Ainv, h->gj_pinv, h->colk, h->rowk);
-        k_gjb_update<<<grid_for(N * N, 256, 16), 256, 0, st>>>(N, k0, nb, h->Ainv, h->gj_pinv, h->colk, h->rowk);
+    const int64_t steps = (N + GJ_NB - 1) / GJ_NB;
+    const bool stepped = N <= GJ_STEP_MAX;
+    // two copies in turn: the last step writes Ainv
+    double *from = stepped && (steps & 1) ? h->Ainv2 : h->Ainv, *to = from == h->Ainv ? h->Ainv2 : h->Ainv;
+    SG_CUDA(cudaMemsetAsync(from, 0, sizeof(double) * N * N, st));
+    const int32_t *row_of = L.Aext ? L.Aext->d_row_of : L.Aown.d_row;
+    SG_B_DISPATCH(L.b, (k_bsr_to_dense<BB, V><<<grid_for(L.Anblk * BB * BB, 256, 16), 256, 0, st>>>(
+                           L.Anblk, row_of, L.d_Acol, A, N, from)));
+    if (stepped) {
+        count_launch((int)steps + 1);
+        double *p0 = h->gj_pinv, *p1 = p0 + GJ_NB * GJ_NB;
+        k_gjb_first<<<1, 256, 0, st>>>(N, (int)std::min<int64_t>(GJ_NB, N), from, p0);
+        for (int64_t K = 0; K < steps; ++K) {
+            k_gjb_step<<<dim3((unsigned)steps, (unsigned)steps), 256, 0, st>>>(N, (int)K, from, to, p0, p1);
+            std::swap(from, to);
+            std::swap(p0, p1);
+        }
+    } else {
+        for (int64_t k0 = 0; k0 < N; k0 += GJ_NB) {
+            const int nb = (int)std::min<int64_t>(GJ_NB, N - k0);
+            count_launch();
+            k_gjb_pivot<<<1, GJ_NB * GJ_NB, 0, st>>>(N, k0, nb, h->Ainv, h->gj_pinv);
+            k_gjb_save<<<grid_for(N * nb, 256), 256, 0, st>>>(N, k0, nb, h->Ainv, h->gj_pinv, h->colk, h->rowk);
+            k_gjb_update<<<grid_for(N * N, 256, 16), 256, 0, st>>>(N, k0, nb, h->Ainv, h->gj_pinv, h->colk, h->rowk);
+        }
     }
     if (h->opt.mixed) k_to_float<<<grid_for(N * N, 256), 256, 0, st>>>(N * N, h->Ainv, h->Ainv32);
     SG_CUDA(cudaGetLastError());
     return SG_OK;
+}
+
+static int numeric_coarsest(sg_amg *h, cudaStream_t st) {
+    return coarsest_inverse<double>(h, level_values(h->L.back()), st);
 }
 
 static int numeric_update(sg_amg *h, cudaStream_t st) {
@@ -1272,20 +1377,8 @@ static int numeric_update32(sg_amg *h, cudaStream_t st) {
                                                                                             L.Dinv, L.Dinv32)));
         SG_CUDA(cudaGetLastError());
         if (l == nl - 1) {
-            const int64_t N = h->nc_dense;
-            SG_CUDA(cudaMemsetAsync(h->Ainv, 0, sizeof(double) * N * N, st));
-            SG_B_DISPATCH(L.b, (k_bsr_to_dense<BB, float><<<grid_for(L.n, 128), 128, 0, st>>>(
-                                   L.n, L.d_Arp, L.d_Acol, L.A32, N, h->Ainv)));
-            for (int64_t k0 = 0; k0 < N; k0 += GJ_NB) {
-                const int nb = (int)std::min<int64_t>(GJ_NB, N - k0);
-                count_launch();
-                k_gjb_pivot<<<1, GJ_NB * GJ_NB, 0, st>>>(N, k0, nb, h->Ainv, h->gj_pinv);
-                k_gjb_save<<<grid_for(N * nb, 256), 256, 0, st>>>(N, k0, nb, h->Ainv, h->gj_pinv, h->colk, h->rowk);
-                k_gjb_update<<<grid_for(N * N, 256, 16), 256, 0, st>>>(N, k0, nb, h->Ainv, h->gj_pinv, h->colk,
-                                                                      h->rowk);
-            }
-            k_to_float<<<grid_for(N * N, 256), 256, 0, st>>>(N * N, h->Ainv, h->Ainv32);
-            SG_CUDA(cudaGetLastError());
+            const int rc = coarsest_inverse<float>(h, L.A32, st);
+            if (rc) return rc;
             break;
         }
         Level &C = h->L[l + 1];
@@ -1374,7 +1467,7 @@ static int make_level(sg_amg *h, const sg_bsr *A0, const std::vector<int32_t> &r
         L.d_Adiag = L.d_diag_own;
         L.Anblk = L.Aown.nblk;
     }
-    if (!rc) rc = alloc_level_buffers(L, h->opt.mixed);
+    if (!rc) rc = alloc_level_buffers(L, h->opt.mixed, h->opt.cheb_degree);
     return rc;
 }
 
@@ -1437,9 +1530,13 @@ static int build_hierarchy(sg_amg *h, const sg_bsr *A0, const double *A0vals, co
                 return set_error(SG_ERR_NUMERIC, "AMG coarsening stalled: coarsest level too large for a dense inverse");
             h->nc_dense = ndof;
             rc = dalloc(&h->Ainv, (size_t)ndof * ndof);
-            if (!rc) rc = dalloc(&h->colk, (size_t)ndof * GJ_NB);
-            if (!rc) rc = dalloc(&h->rowk, (size_t)ndof * GJ_NB);
-            if (!rc) rc = dalloc(&h->gj_pinv, (size_t)GJ_NB * GJ_NB);
+            if (ndof <= GJ_STEP_MAX) {
+                if (!rc) rc = dalloc(&h->Ainv2, (size_t)ndof * ndof);
+            } else {
+                if (!rc) rc = dalloc(&h->colk, (size_t)ndof * GJ_NB);
+                if (!rc) rc = dalloc(&h->rowk, (size_t)ndof * GJ_NB);
+            }
+            if (!rc) rc = dalloc(&h->gj_pinv, (size_t)2 * GJ_NB * GJ_NB);
             if (!rc && o.mixed) rc = dalloc(&h->Ainv32, (size_t)ndof * ndof);
             return rc;
         }
@@ -1507,10 +1604,33 @@ static int level_residual(Level &L, LevelView<T> &v, cudaStream_t st) {
     return rect_spmv<T, T>(L.b, L.b, L.n, L.d_Arp, L.d_Acol, v.A, v.x, v.r, 1.0, 0.0, v.rhs, 1, st, L.Anblk);
 }
 
+// Whether a level's Chebyshev steps run as the epilogue of their residual.  They then alternate
+// between x and the residual's array r (free while smoothing); the first array of a run of
+// steps is chosen so that the last one writes x.  The FP16 copy of level 0 has its own residual kernel.
+template <typename T>
+static bool fused_smoother(const Level &L) {
+    return !(std::is_same<T, float>::value && L.A16);
+}
+
+// The smoothing steps of one side of the cycle.  x_zero (before the coarse correction): from x = 0;
+// otherwise from the array that holds x: v.x, or (fused, odd degree) v.r.
 template <typename T>
 static int smooth(sg_amg *h, Level &L, LevelView<T> &v, bool x_zero, cudaStream_t st) {
     const int deg = h->opt.cheb_degree;
     int rc = SG_OK;
+    if (fused_smoother<T>(L)) {
+        const int steps = x_zero ? deg - 1 : deg;          // steps with a residual
+        T *cur = (steps & 1) ? v.r : v.x, *other = cur == v.x ? v.r : v.x;
+        if (x_zero)
+            SG_B_DISPATCH(L.b, (k_cheb<BB, T><<<grid_for(L.n, 256), 256, 0, st>>>(L.n, 0, L.coef, v.Dinv, v.rhs, v.d, cur, 1)));
+        for (int k = deg - steps; k < deg && !rc; ++k) {
+            rc = cheb_step<T>(L.b, L.n, L.Anblk, L.d_Arp, L.d_Acol, v.A, cur, v.rhs,
+                              ChebStep<T>{L.coef + 2 * k, v.Dinv, v.d, other, k == 0}, st);
+            std::swap(cur, other);
+        }
+        SG_CUDA(cudaGetLastError());
+        return rc;
+    }
     for (int k = 0; k < deg && !rc; ++k) {
         const T *r = v.rhs;
         if (!(x_zero && k == 0)) {
@@ -1519,16 +1639,19 @@ static int smooth(sg_amg *h, Level &L, LevelView<T> &v, bool x_zero, cudaStream_
             r = v.r;
         }
         const int xz = (x_zero && k == 0) ? 1 : 0;
-        SG_B_DISPATCH(L.b, (k_cheb<BB, T><<<grid_for(L.n, 256), 256, 0, st>>>(L.n, k, h->opt.cheb_ratio, L.lmax, v.Dinv, r, v.d, v.x, xz)));
+        SG_B_DISPATCH(L.b, (k_cheb<BB, T><<<grid_for(L.n, 256), 256, 0, st>>>(L.n, k, L.coef, v.Dinv, r, v.d, v.x, xz)));
     }
     SG_CUDA(cudaGetLastError());
     return rc;
 }
 
+// rhs0, x0: level 0's right-hand side and result in place of its own arrays (the caller's vectors)
 template <typename T>
-static int vcycle(sg_amg *h, int l, cudaStream_t st) {
+static int vcycle(sg_amg *h, int l, cudaStream_t st, const T *rhs0 = nullptr, T *x0 = nullptr) {
     Level &L = h->L[l];
     LevelView<T> v = view<T>(L);
+    if (rhs0) v.rhs = const_cast<T *>(rhs0);   // read only
+    if (x0) v.x = x0;
     if (l == (int)h->L.size() - 1) {
         const T *M = std::is_same<T, float>::value ? (const T *)h->Ainv32 : (const T *)h->Ainv;
         k_dense_gemv<T><<<grid_for(h->nc_dense * 32, 256), 256, 0, st>>>(h->nc_dense, M, v.rhs, v.x);
@@ -1541,7 +1664,10 @@ static int vcycle(sg_amg *h, int l, cudaStream_t st) {
     if (!rc) rc = level_residual<T>(L, v, st);
     if (!rc) rc = rect_spmv<T, T>(L.bc, L.b, C.n, L.R.d_rp, L.R.d_col, v.R, v.r, c.rhs, 1.0, 0.0, nullptr, 0, st, L.R.nblk);
     if (!rc) rc = vcycle<T>(h, l + 1, st);
-    if (!rc) rc = rect_spmv<T, T>(L.b, L.bc, L.n, L.P.d_rp, L.P.d_col, v.P, c.x, v.x, 1.0, 1.0, nullptr, 0, st, L.P.nblk);
+    // x + P e to where the smoother starts from
+    T *to = fused_smoother<T>(L) && (h->opt.cheb_degree & 1) ? v.r : v.x;
+    if (!rc) rc = rect_spmv<T, T>(L.b, L.bc, L.n, L.P.d_rp, L.P.d_col, v.P, c.x, to, 1.0, 1.0, v.x, to == v.x ? 0 : 3, st,
+                                  L.P.nblk);
     if (!rc) rc = smooth<T>(h, L, v, false, st);
     return rc;
 }
@@ -1581,7 +1707,7 @@ extern "C" int sg_amg_create(const sg_bsr *A, const double *A_vals, const double
     if (!rc) rc = build_hierarchy(h, A, A_vals, nullspace, nns, fixed, as_stream(stream));
     if (rc) {
         for (auto &L : h->L) free_level(L);
-        cudaFree(h->Ainv); cudaFree(h->Ainv32); cudaFree(h->colk); cudaFree(h->rowk); cudaFree(h->dots);
+        cudaFree(h->Ainv); cudaFree(h->Ainv2); cudaFree(h->Ainv32); cudaFree(h->colk); cudaFree(h->rowk); cudaFree(h->dots);
         cudaFree(h->gj_pinv);
         delete h;
         return rc;
@@ -1606,6 +1732,7 @@ extern "C" int sg_amg_destroy(sg_amg *h) {
     }
     for (auto &L : h->L) free_level(L);
     cudaFree(h->Ainv);
+    cudaFree(h->Ainv2);
     cudaFree(h->Ainv32);
     cudaFree(h->colk);
     cudaFree(h->rowk);
@@ -1711,15 +1838,17 @@ extern "C" int sg_amg_apply(sg_amg *h, const double *r, double *z, void *stream)
         }
         if (!rc) k_to_double<<<grid_for(nd, 256), 256, 0, st>>>(nd, L.x32, z);
     } else {
-        SG_CUDA(cudaMemcpyAsync(L.rhs, r, sizeof(double) * nd, cudaMemcpyDeviceToDevice, st));
-        rc = vcycle<double>(h, 0, st);
+        const double *b = r;
+        if (z < r + nd && r < z + nd) {   // they share memory: the cycle needs the right-hand side to its end
+            SG_CUDA(cudaMemcpyAsync(L.rhs, r, sizeof(double) * nd, cudaMemcpyDeviceToDevice, st));
+            b = L.rhs;
+        }
+        rc = vcycle<double>(h, 0, st, b, z);
         if (!rc && h->corr_on) {
             LevelView<double> v = view<double>(L);
-            rc = rect_spmv<double, double>(L.b, L.b, L.n, L.d_Arp, L.d_Acol, v.A, L.x, L.r, 1.0, 0.0, L.rhs, 1, st,
-                                           L.Anblk);
-            if (!rc) k_corr_apply<double><<<grid_for(L.n, 256), 256, 0, st>>>(L.n, h->corrC, L.r, L.x);
+            rc = rect_spmv<double, double>(L.b, L.b, L.n, L.d_Arp, L.d_Acol, v.A, z, L.r, 1.0, 0.0, b, 1, st, L.Anblk);
+            if (!rc) k_corr_apply<double><<<grid_for(L.n, 256), 256, 0, st>>>(L.n, h->corrC, L.r, z);
         }
-        if (!rc) SG_CUDA(cudaMemcpyAsync(z, L.x, sizeof(double) * nd, cudaMemcpyDeviceToDevice, st));
     }
     SG_CUDA(cudaGetLastError());
     return rc;

@@ -25,20 +25,56 @@ template <> struct Acc<float> { using type = float; };
 // k_spmv_blk: G lanes per block row of the matrix, one block per lane per step (the lane reads
 //   the block's br*bc contiguous values).  Best for 3x3 (G = 32 at ~28 blocks per row:
 //   4.8 TB/s) and the short rows of P.
+//   What bounds the fine one is the L1 data pipe: nine value loads of a lane at a 36- or 72-byte
+//   stride (28.3M blocks: FP32 0.266 ms, 4.3 TB/s; FP64 0.398 ms, 5.6 TB/s).  Copying a CTA's values to
+//   shared memory by 16-byte cp.async, columns and x gathered meanwhile, removes those requests
+//   but waits longer than it saves (0.41 and 0.55 ms).
 // k_spmv_row: LPR lanes per block row of the matrix, BR lanes per block: lane (slot, a) reads
 //   row a of the group's slot-th block, so a warp's loads walk one contiguous run of SLOTS
 //   blocks; U steps are loaded before the first product.  Best for wide blocks (6x6: 2.3x
 //   the lane-per-block mapping, whose 288-byte lane stride spreads each load over 32 lines).
 // Both sum in a fixed order (reproducible bitwise from run to run).
-template <int BR, int BC, int G, typename VT, typename XT>
+// One Chebyshev step on D^-1 A as the epilogue of a residual product: r = b - A x stays in
+// registers, d = c1 d + c2 D^-1 r, x_new = x + d (x_new another array than x, whose old entries
+// other rows still gather).  The same operations as a residual kernel followed by k_cheb.
+template <int B, typename T>
+struct ChebRow {
+    T b[B], di[B], d, x;
+    __device__ __forceinline__ void load(const ChebStep<T> &s, const T *__restrict__ bvec, const T *__restrict__ xv,
+                                         int64_t row, int a) {
+#pragma unroll
+        for (int c = 0; c < B; ++c) {
+            b[c] = bvec[row * B + c];
+            di[c] = s.dinv[(row * B + a) * B + c];
+        }
+        d = s.first ? (T)0 : s.d[row * B + a];
+        x = xv[row * B + a];
+    }
+    __device__ __forceinline__ void store(const ChebStep<T> &s, const T (&r)[B], int64_t row, int a) const {
+        T t = 0;
+#pragma unroll
+        for (int c = 0; c < B; ++c) t += di[c] * r[c];
+        const T dn = s.first ? (T)s.coef[1] * t : (T)s.coef[0] * d + (T)s.coef[1] * t;
+        s.d[row * B + a] = dn;
+        s.xn[row * B + a] = x + dn;
+    }
+};
+
+// rows of a CTA of k_spmv_blk: four per warp slot
+#define SPMV_MAX_ROWS(G) (32 * (32 / (G)))
+template <int BR, int BC, int G, typename VT, typename XT, bool CHEB = false>
 __global__ void __launch_bounds__(256) k_spmv_blk(int64_t nrows, const int32_t *__restrict__ rp,
                                                   const int32_t *__restrict__ col, const VT *__restrict__ vals,
                                                   const XT *__restrict__ x, XT *__restrict__ y, double alpha,
                                                   double beta, const XT *__restrict__ bvec, int mode,
-                                                  int64_t rows_per_cta) {
+                                                  int64_t rows_per_cta, const ChebStep<XT> cheb = {}) {
     using A = typename Acc<XT>::type;
     constexpr int GPW = 32 / G;  // rows per warp
     const int lane = threadIdx.x & 31, g = lane / G, gl = lane - g * G;
+    // CHEB: the sums of the CTA's rows, for the step over all of them after the products (the
+    // step's loads then run along the rows; as an epilogue of each row they took more of the L1
+    // pipe than the vector kernel they replace, and the registers of a quarter of the warps)
+    __shared__ A sums[CHEB ? SPMV_MAX_ROWS(G) * BR : 1];
     // a CTA owns rows_per_cta consecutive rows and its warps walk them in order, so the x
     // entries of neighbouring rows are still in L1 when the next rows gather them
     const int64_t r0 = (int64_t)blockIdx.x * rows_per_cta;
@@ -67,23 +103,42 @@ __global__ void __launch_bounds__(256) k_spmv_blk(int64_t nrows, const int32_t *
         for (int off = G / 2; off > 0; off >>= 1)
 #pragma unroll
             for (int a = 0; a < BR; ++a) acc[a] += __shfl_xor_sync(0xffffffffu, acc[a], off);
-        if (row < rend && gl == 0) {
+        if (CHEB) {
+            if (row < rend && gl == 0)
+#pragma unroll
+                for (int a = 0; a < BR; ++a) sums[(int)(row - r0) * BR + a] = acc[a];
+        } else if (row < rend && gl == 0) {
 #pragma unroll
             for (int a = 0; a < BR; ++a) {
                 const int64_t k = row * BR + a;
                 if (mode == 1) y[k] = (XT)((A)bvec[k] - acc[a]);
+                else if (mode == 3) y[k] = (XT)(alpha * acc[a] + beta * (A)bvec[k]);
                 else if (beta == 0.0) y[k] = (XT)(alpha * acc[a]);
                 else y[k] = (XT)(alpha * acc[a] + beta * (A)y[k]);
             }
         }
     }
+    if constexpr (CHEB) {
+        __syncthreads();
+        for (int e = threadIdx.x; e < (int)(rend - r0) * BR; e += blockDim.x) {
+            const int lr = e / BR, a = e - lr * BR;
+            const int64_t row = r0 + lr;
+            ChebRow<BR, XT> own;
+            own.load(cheb, bvec, x, row, a);
+            XT r[BR];
+#pragma unroll
+            for (int c = 0; c < BR; ++c) r[c] = (XT)((A)own.b[c] - sums[lr * BR + c]);
+            own.store(cheb, r, row, a);
+        }
+    }
 }
 
-template <int BR, int BC, int LPR, int U, typename VT, typename XT>
+template <int BR, int BC, int LPR, int U, typename VT, typename XT, bool CHEB = false>
 __global__ void __launch_bounds__(256) k_spmv_row(int64_t nrows, const int32_t *__restrict__ rp,
                                                   const int32_t *__restrict__ col, const VT *__restrict__ vals,
                                                   const XT *__restrict__ x, XT *__restrict__ y, double alpha,
-                                                  double beta, const XT *__restrict__ bvec, int mode) {
+                                                  double beta, const XT *__restrict__ bvec, int mode,
+                                                  const ChebStep<XT> cheb = {}) {
     using A = typename Acc<XT>::type;
     constexpr int BB = BR * BC, SLOTS = LPR / BR, RPW = 32 / LPR;  // rows per warp
     const int lane = threadIdx.x & 31, rg = lane / LPR, li = lane - rg * LPR;
@@ -94,6 +149,8 @@ __global__ void __launch_bounds__(256) k_spmv_row(int64_t nrows, const int32_t *
     for (int64_t base = warp * RPW; base < nrows; base += nwarps * RPW) {
         const int64_t row = base + rg;
         A acc = 0;
+        ChebRow<BR, XT> own;
+        if (CHEB && row < nrows && active && slot == 0) own.load(cheb, bvec, x, row, a);
         if (row < nrows && active) {
             const int32_t p0 = rp[row] + slot, p1 = rp[row + 1];
             for (int32_t p = p0; p < p1; p += U * SLOTS) {
@@ -130,9 +187,16 @@ __global__ void __launch_bounds__(256) k_spmv_row(int64_t nrows, const int32_t *
         const int g0 = rg * LPR;
 #pragma unroll
         for (int sl = 0; sl < SLOTS; ++sl) tot += __shfl_sync(0xffffffffu, acc, g0 + sl * BR + (active ? a : 0));
-        if (row < nrows && active && slot == 0) {
+        if (CHEB) {
+            XT r[BR];
+            const XT ra = row < nrows && active && slot == 0 ? (XT)((A)own.b[a] - tot) : (XT)0;
+#pragma unroll
+            for (int c = 0; c < BR; ++c) r[c] = __shfl_sync(0xffffffffu, ra, g0 + c);
+            if (row < nrows && active && slot == 0) own.store(cheb, r, row, a);
+        } else if (row < nrows && active && slot == 0) {
             const int64_t k = row * BR + a;
             if (mode == 1) y[k] = (XT)((A)bvec[k] - tot);
+            else if (mode == 3) y[k] = (XT)(alpha * tot + beta * (A)bvec[k]);
             else if (beta == 0.0) y[k] = (XT)(alpha * tot);
             else y[k] = (XT)(alpha * tot + beta * (A)y[k]);
         }
@@ -144,11 +208,12 @@ __global__ void __launch_bounds__(256) k_spmv_row(int64_t nrows, const int32_t *
 // walks its row serially).  Each warp uses k_spmv_row's (slot, a) lane mapping over its share
 // of the row (warp w starts at slot w * SLOTS and steps by W * SLOTS); the warps' partial sums
 // meet in shared memory and are added in warp order (reproducible bitwise).
-template <int BR, int BC, int W, typename VT, typename XT>
+template <int BR, int BC, int W, typename VT, typename XT, bool CHEB = false>
 __global__ void __launch_bounds__(32 * W) k_spmv_cta(int64_t nrows, const int32_t *__restrict__ rp,
                                                      const int32_t *__restrict__ col, const VT *__restrict__ vals,
                                                      const XT *__restrict__ x, XT *__restrict__ y, double alpha,
-                                                     double beta, const XT *__restrict__ bvec, int mode) {
+                                                     double beta, const XT *__restrict__ bvec, int mode,
+                                                     const ChebStep<XT> cheb = {}) {
     using A = typename Acc<XT>::type;
     constexpr int BB = BR * BC, SLOTS = 32 / BR;
     __shared__ A part[W][BR];
@@ -157,6 +222,8 @@ __global__ void __launch_bounds__(32 * W) k_spmv_cta(int64_t nrows, const int32_
     const bool active = slot < SLOTS;
     for (int64_t row = blockIdx.x; row < nrows; row += gridDim.x) {
         A acc = 0;
+        ChebRow<BR, XT> own;
+        if (CHEB && w == 0 && lane < BR) own.load(cheb, bvec, x, row, lane);
         if (active) {
             const int32_t p1 = rp[row + 1];
             for (int32_t p = rp[row] + w * SLOTS + slot; p < p1; p += W * SLOTS) {
@@ -172,12 +239,25 @@ __global__ void __launch_bounds__(32 * W) k_spmv_cta(int64_t nrows, const int32_
         for (int sl = 0; sl < SLOTS; ++sl) tot += __shfl_sync(0xffffffffu, acc, sl * BR + (active ? a : 0));
         if (lane < BR) part[w][lane] = tot;
         __syncthreads();
-        if (w == 0 && lane < BR) {
+        if (CHEB) {
+            if (w == 0) {
+                A sum = 0;
+                if (lane < BR)
+#pragma unroll
+                    for (int q = 0; q < W; ++q) sum += part[q][lane];
+                XT r[BR];
+                const XT ra = lane < BR ? (XT)((A)own.b[lane < BR ? lane : 0] - sum) : (XT)0;
+#pragma unroll
+                for (int c = 0; c < BR; ++c) r[c] = __shfl_sync(0xffffffffu, ra, c);
+                if (lane < BR) own.store(cheb, r, row, lane);
+            }
+        } else if (w == 0 && lane < BR) {
             A sum = 0;
 #pragma unroll
             for (int q = 0; q < W; ++q) sum += part[q][lane];
             const int64_t k = row * BR + lane;
             if (mode == 1) y[k] = (XT)((A)bvec[k] - sum);
+            else if (mode == 3) y[k] = (XT)(alpha * sum + beta * (A)bvec[k]);
             else if (beta == 0.0) y[k] = (XT)(alpha * sum);
             else y[k] = (XT)(alpha * sum + beta * (A)y[k]);
         }
@@ -188,9 +268,10 @@ __global__ void __launch_bounds__(32 * W) k_spmv_cta(int64_t nrows, const int32_
 // rows below which a coarse 6x6 level with long rows takes a CTA per row (k_spmv_cta)
 constexpr int64_t CTA_ROW_LIMIT = 1184;
 
-template <int BR, int BC, typename VT, typename XT>
+template <int BR, int BC, bool CHEB = false, typename VT, typename XT>
 static void spmv_launch(int64_t nrows, int64_t nblk, const int32_t *rp, const int32_t *col, const VT *vals,
-                        const XT *x, XT *y, double alpha, double beta, const XT *bvec, int mode, cudaStream_t st) {
+                        const XT *x, XT *y, double alpha, double beta, const XT *bvec, int mode, cudaStream_t st,
+                        const ChebStep<XT> &cheb = {}) {
     const double avg = nblk > 0 && nrows > 0 ? (double)nblk / (double)nrows : 8.0;
     // the node-block shapes of the fine level are the ones timed for the roofline report
     constexpr bool fine = (BR == BC) && (BR == 3 || BR == 2);
@@ -201,8 +282,8 @@ static void spmv_launch(int64_t nrows, int64_t nblk, const int32_t *rp, const in
     if constexpr (wide) {
         if (nrows < CTA_ROW_LIMIT && avg >= 48.0) {
             count_launch();
-            k_spmv_cta<BR, BC, 8, VT, XT><<<(unsigned)nrows, 256, 0, st>>>(nrows, rp, col, vals, x, y, alpha, beta,
-                                                                           bvec, mode);
+            k_spmv_cta<BR, BC, 8, VT, XT, CHEB><<<(unsigned)nrows, 256, 0, st>>>(nrows, rp, col, vals, x, y, alpha, beta,
+                                                                                 bvec, mode, cheb);
             return;
         }
     }
@@ -210,20 +291,20 @@ static void spmv_launch(int64_t nrows, int64_t nblk, const int32_t *rp, const in
         const int lpr = avg >= 48.0 ? 32 : 16;
         const unsigned grid = grid_for(nrows * lpr, 256, 16);
         if (lpr == 32) {
-            if (wide) k_spmv_row<BR, BC, 32, 1, VT, XT><<<grid, 256, 0, st>>>(nrows, rp, col, vals, x, y, alpha, beta, bvec, mode);
+            if (wide) k_spmv_row<BR, BC, 32, 1, VT, XT, CHEB><<<grid, 256, 0, st>>>(nrows, rp, col, vals, x, y, alpha, beta, bvec, mode, cheb);
             else k_spmv_row<BR, BC, 32, 3, VT, XT><<<grid, 256, 0, st>>>(nrows, rp, col, vals, x, y, alpha, beta, bvec, mode);
         } else {
-            k_spmv_row<BR, BC, 16, 2, VT, XT><<<grid, 256, 0, st>>>(nrows, rp, col, vals, x, y, alpha, beta, bvec, mode);
+            k_spmv_row<BR, BC, 16, 2, VT, XT, CHEB><<<grid, 256, 0, st>>>(nrows, rp, col, vals, x, y, alpha, beta, bvec, mode, cheb);
         }
     } else {
         const int G = avg >= 16.0 ? 32 : (avg >= 8.0 ? 16 : 8);
         // up to four rows (G = 32) or 16 rows (G = 8) per warp
-        const int64_t rpc = chunk_len(nrows, 8 * (32 / G), 32 * (32 / G));
+        const int64_t rpc = chunk_len(nrows, 8 * (32 / G), SPMV_MAX_ROWS(G));
         const unsigned grid = grid_chunks(nrows, rpc);
         switch (G) {
-            case 32: k_spmv_blk<BR, BC, 32, VT, XT><<<grid, 256, 0, st>>>(nrows, rp, col, vals, x, y, alpha, beta, bvec, mode, rpc); break;
-            case 16: k_spmv_blk<BR, BC, 16, VT, XT><<<grid, 256, 0, st>>>(nrows, rp, col, vals, x, y, alpha, beta, bvec, mode, rpc); break;
-            default: k_spmv_blk<BR, BC, 8, VT, XT><<<grid, 256, 0, st>>>(nrows, rp, col, vals, x, y, alpha, beta, bvec, mode, rpc); break;
+            case 32: k_spmv_blk<BR, BC, 32, VT, XT, CHEB><<<grid, 256, 0, st>>>(nrows, rp, col, vals, x, y, alpha, beta, bvec, mode, rpc, cheb); break;
+            case 16: k_spmv_blk<BR, BC, 16, VT, XT, CHEB><<<grid, 256, 0, st>>>(nrows, rp, col, vals, x, y, alpha, beta, bvec, mode, rpc, cheb); break;
+            default: k_spmv_blk<BR, BC, 8, VT, XT, CHEB><<<grid, 256, 0, st>>>(nrows, rp, col, vals, x, y, alpha, beta, bvec, mode, rpc, cheb); break;
         }
     }
     if (fine) instr_end(tk, st);
@@ -246,6 +327,24 @@ template int rect_spmv<float, float>(int, int, int64_t, const int32_t *, const i
 template int rect_spmv<float, double>(int, int, int64_t, const int32_t *, const int32_t *, const float *,
                                       const double *, double *, double, double, const double *, int, cudaStream_t,
                                       int64_t);
+
+template <typename T>
+int cheb_step(int b, int64_t nrows, int64_t nblk, const int32_t *rp, const int32_t *col, const T *vals, const T *x,
+              const T *rhs, const ChebStep<T> &step, cudaStream_t st) {
+#define SG_CHEB_CASE(R)                                                                                       \
+    if (b == R) {                                                                                             \
+        spmv_launch<R, R, true>(nrows, nblk, rp, col, vals, x, (T *)nullptr, 1.0, 0.0, rhs, 1, st, step);     \
+        SG_CUDA(cudaGetLastError());                                                                          \
+        return SG_OK;                                                                                         \
+    }
+    SG_CHEB_CASE(1) SG_CHEB_CASE(2) SG_CHEB_CASE(3) SG_CHEB_CASE(6)
+#undef SG_CHEB_CASE
+    return set_error(SG_ERR_ARG, "unsupported BSR block shape");
+}
+template int cheb_step<double>(int, int64_t, int64_t, const int32_t *, const int32_t *, const double *, const double *,
+                               const double *, const ChebStep<double> &, cudaStream_t);
+template int cheb_step<float>(int, int64_t, int64_t, const int32_t *, const int32_t *, const float *, const float *,
+                              const float *, const ChebStep<float> &, cudaStream_t);
 
 template <typename VT, typename XT>
 int bsr_spmv(const sg_bsr &A, const VT *vals, const XT *x, XT *y, double alpha, double beta, cudaStream_t st) {

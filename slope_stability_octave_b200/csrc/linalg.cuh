@@ -15,12 +15,27 @@ int bsr_spmv(const sg_bsr &A, const VT *vals, const XT *x, XT *y, double alpha, 
 template <typename VT, typename XT>
 int bsr_residual(const sg_bsr &A, const VT *vals, const XT *x, const XT *b, XT *r, cudaStream_t st);
 
-// Rectangular-block row SpMV: y = alpha * M x + beta * y (mode 0) or y = bvec - M x (mode 1),
+// Rectangular-block row SpMV: y = alpha * M x + beta * y (mode 0) y = bvec - M x (mode 1)
+// or y = alpha * M x + beta * bvec (mode 3),
 // M with br x bc blocks.  Supported shapes: 1x1 2x2 3x3 6x6 2x3 3x2 3x6 6x3.
 // nblk (total blocks, -1 if unknown) selects the number of lanes per row.
 template <typename VT, typename XT>
 int rect_spmv(int br, int bc, int64_t nrows, const int32_t *rp, const int32_t *col, const VT *vals, const XT *x,
               XT *y, double alpha, double beta, const XT *bvec, int mode, cudaStream_t st, int64_t nblk = -1);
+
+// One Chebyshev smoothing step in one kernel: r = rhs - A x (not stored), d = c1 d + c2 D^-1 r (first:
+// d = c2 D^-1 r), xn = x + d, with coef = {c1, c2} on the device and D^-1 as b x b blocks; xn and x
+// are different arrays.  Bitwise the same as rect_spmv's residual followed by the vector step.
+template <typename T>
+struct ChebStep {
+    const double *coef;
+    const T *dinv;
+    T *d, *xn;
+    int first;
+};
+template <typename T>
+int cheb_step(int b, int64_t nrows, int64_t nblk, const int32_t *rp, const int32_t *col, const T *vals, const T *x,
+              const T *rhs, const ChebStep<T> &step, cudaStream_t st);
 
 // Y(:, c) = A X(:, c) for c < k, FP64 3x3 blocks; X, Y column-major (leading dimensions may
 // be negative).  Reads the matrix once per 8 columns; each column equals bsr_spmv's bitwise.
