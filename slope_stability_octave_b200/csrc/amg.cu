@@ -721,6 +721,255 @@ __global__ void k_gather_Ac_warp(int64_t nitems, const int32_t *__restrict__ qma
     }
 }
 
+// Team form of the two gathers for 3 x 6 blocks (the fine level of an elasticity hierarchy):
+// B * BC / 2 = 9 lanes form one output block.  Lane (m, h) of a team takes row m of the
+// right-hand block, columns 2h and 2h + 1, so a team reads that block in one request of
+// contiguous 8- or 16-byte parts, and sums its m's share of the products; the shares meet in B - 1
+// rotations.
+template <typename V> struct Pair2;
+template <> struct Pair2<double> { using type = double2; };
+template <> struct Pair2<float> { using type = float2; };
+
+template <int B, int BC> struct Team {
+    static constexpr int H = BC / 2, LANES = B * H, PER_WARP = 32 / LANES;
+    int team, e, m, h, base;
+    bool on;
+    __device__ Team(int lane) {
+        team = lane / LANES;
+        on = team < PER_WARP;
+        e = lane - team * LANES;
+        m = e / H;
+        h = e - m * H;
+        base = team * LANES;
+    }
+    // lane holding (m - k mod B, h)
+    __device__ int from(int k) const {
+        const int mm = m >= k ? m - k : m - k + B;
+        return on ? base + mm * H + h : 0;
+    }
+    // acc[r][2] of every lane summed over the team's m's: lane m returns rows m, m + B, ...
+    template <int ROWS, typename T>
+    __device__ void reduce(const T (&acc)[ROWS][2], T (&out)[ROWS / B][2]) const {
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+            const int want = m + k >= B ? m + k - B : m + k;   // the row the receiving lane owns
+#pragma unroll
+            for (int q = 0; q < ROWS / B; ++q)
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    T v = acc[q * B][s];
+#pragma unroll
+                    for (int r = 1; r < B; ++r) v = want == r ? acc[q * B + r][s] : v;
+                    if (k == 0) out[q][s] = v;
+                    else out[q][s] += __shfl_sync(0xffffffffu, v, from(k));
+                }
+        }
+    }
+    // the same block summed by all teams of the warp: the first team returns the sum
+    template <int N, typename T> __device__ void join(T (&v)[N][2]) const {
+#pragma unroll
+        for (int q = 0; q < N; ++q)
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                T sum = v[q][s];
+#pragma unroll
+                for (int t = 1; t < PER_WARP; ++t) sum += __shfl_sync(0xffffffffu, v[q][s], t * LANES + e < 32 ? t * LANES + e : 0);
+                v[q][s] = sum;
+            }
+    }
+};
+
+// A P on its plan's pattern, a team per output block.  A CTA takes a run of output blocks; the matrix
+// blocks of their rows and their pair indices are contiguous, so both are copied to shared memory,
+// and a pair costs one gather of P, unrolled five deep.  Runs that exceed the shared arrays are
+// halved; a single output block that does is summed from global memory.
+// What bounds it: P's sectors from L2 (39M pairs of 144 bytes: 7 TB/s).  A thread per output block, each
+// lane reading its own P block, kept the L1 tags busy instead: FP64 39M pairs 1.57 -> 1.04 ms, FP32
+// 4.23 -> 3.13 ms on the layered slope.  Runs of 32 or 96 blocks, or A read in place, are slower
+// (1.12 to 1.2 ms); the same form of the prolongator's A T, whose pairs read A once, gains
+// nothing in FP32.
+constexpr int TP_RUN = 64;                 // output blocks of a CTA
+constexpr int TP_PAIRS = 20 * TP_RUN;
+constexpr int TP_BLOCKS = 4 * TP_RUN;
+
+template <int B, int BC, typename V>
+__global__ void __launch_bounds__(128) k_team_AP(int64_t nblk, const int32_t *__restrict__ row,
+                                                 const int32_t *__restrict__ Arp, const int64_t *__restrict__ lptr,
+                                                 const int32_t *__restrict__ la, const int32_t *__restrict__ lb,
+                                                 const V *__restrict__ A, const V *__restrict__ P, V *__restrict__ AP) {
+    using T = typename GAcc<V>::type;
+    using V2 = typename Pair2<V>::type;
+    using Tm = Team<B, BC>;
+    constexpr int U = 5, TEAMS = 4 * Tm::PER_WARP;
+    __shared__ V sA[TP_BLOCKS * B * B];
+    __shared__ int2 sI[TP_PAIRS];
+    const Tm tm(threadIdx.x & 31);
+    const int64_t end = ((int64_t)blockIdx.x + 1) * TP_RUN < nblk ? ((int64_t)blockIdx.x + 1) * TP_RUN : nblk;
+    for (int64_t q0 = (int64_t)blockIdx.x * TP_RUN, q1; q0 < end; q0 = q1) {
+        const int64_t a0 = Arp[row[q0]], p0 = lptr[q0];
+        int na, np;
+        for (q1 = end;; q1 = q0 + (q1 - q0) / 2) {
+            const int64_t wa = Arp[row[q1 - 1] + 1] - a0, wp = lptr[q1] - p0;
+            na = wa <= TP_BLOCKS ? (int)wa : -1;
+            np = wp <= TP_PAIRS ? (int)wp : -1;
+            if ((na >= 0 && np >= 0) || q1 == q0 + 1) break;
+        }
+        const bool staged = na >= 0 && np >= 0;
+        if (staged) {
+            const V *src = A + a0 * B * B;
+#pragma unroll 4
+            for (int t = threadIdx.x; t < na * B * B; t += 128) sA[t] = __ldg(src + t);
+#pragma unroll 4
+            for (int t = threadIdx.x; t < np; t += 128)
+                sI[t] = make_int2((int)(la[p0 + t] - a0), lb[p0 + t]);
+        }
+        __syncthreads();
+        for (int64_t w0 = q0 + (threadIdx.x >> 5) * Tm::PER_WARP; w0 < q1; w0 += TEAMS) {
+            const int64_t q = w0 + tm.team;
+            const bool live = tm.on && q < q1;
+            T acc[B][2];
+#pragma unroll
+            for (int r = 0; r < B; ++r) acc[r][0] = acc[r][1] = 0;
+            if (live) {
+                if (staged) {
+                    const int l1 = (int)(lptr[q + 1] - p0);
+                    for (int l = (int)(lptr[q] - p0); l < l1; l += U) {
+                        V2 x[U];
+                        int ka[U];
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            const int2 k = sI[l + u < l1 ? l + u : l1 - 1];
+                            ka[u] = k.x * B * B + tm.m;
+                            x[u] = __ldg(reinterpret_cast<const V2 *>(P + (int64_t)k.y * B * BC) + tm.e);
+                        }
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            if (u > 0 && l + u >= l1) x[u].x = x[u].y = 0;
+#pragma unroll
+                            for (int r = 0; r < B; ++r) {
+                                const T av = (T)sA[ka[u] + r * B];
+                                acc[r][0] += av * (T)x[u].x;
+                                acc[r][1] += av * (T)x[u].y;
+                            }
+                        }
+                    }
+                } else {
+                    for (int64_t l = lptr[q]; l < lptr[q + 1]; ++l) {
+                        const int64_t a = la[l], k = lb[l];
+                        const V2 x = __ldg(reinterpret_cast<const V2 *>(P + k * B * BC) + tm.e);
+#pragma unroll
+                        for (int r = 0; r < B; ++r) {
+                            const T av = (T)A[a * B * B + r * B + tm.m];
+                            acc[r][0] += av * (T)x.x;
+                            acc[r][1] += av * (T)x.y;
+                        }
+                    }
+                }
+            }
+            __syncwarp();
+            T s[1][2];
+            tm.template reduce<B, T>(acc, s);       // row m of the block
+            V2 w;
+            w.x = (V)s[0][0];
+            w.y = (V)s[0][1];
+            if (live) reinterpret_cast<V2 *>(AP + q * B * BC)[tm.e] = w;
+        }
+        __syncthreads();
+    }
+}
+
+// P'(A P), a warp per output block (about 63 pairs on the SSR hierarchy): its teams split the pairs.
+// Lane (m, h) multiplies row m of the P block with its part of the AP block.  The pair indices of
+// a team are read a batch at a time and handed round by shuffles; U pairs are in flight.
+// What bounds it: latency of the gathers, with AP read back from DRAM several times.  Against lane
+// groups that read whole blocks per lane: FP64 10.6M pairs 0.98 -> 0.73 ms, FP32 on the layered
+// slope 2.17 -> 1.52 ms.  FP64 with U = 3 holds 96 registers (0.92 ms); a team per output block
+// without the split is limited by the longest list of a warp (1.83 ms).
+template <int B, int BC, typename V>
+__global__ void __launch_bounds__(128) k_team_Ac(int64_t nitems, const int32_t *__restrict__ qmap,
+                                                 const int32_t *__restrict__ row, const int32_t *__restrict__ col,
+                                                 const int64_t *__restrict__ lptr, const int32_t *__restrict__ la,
+                                                 const int32_t *__restrict__ lb, const V *__restrict__ P,
+                                                 const V *__restrict__ AP, const uint8_t *__restrict__ dead,
+                                                 V *__restrict__ Ac, int64_t chunk) {
+    using T = typename GAcc<V>::type;
+    using V2 = typename Pair2<V>::type;
+    using Tm = Team<B, BC>;
+    constexpr int U = sizeof(V) == 8 ? 2 : 5;
+    const Tm tm(threadIdx.x & 31);
+    const int64_t c0 = (int64_t)blockIdx.x * chunk, c1 = c0 + chunk < nitems ? c0 + chunk : nitems;
+    for (int64_t it = c0 + (threadIdx.x >> 5); it < c1; it += blockDim.x >> 5) {
+        T acc[BC][2];
+#pragma unroll
+        for (int r = 0; r < BC; ++r) acc[r][0] = acc[r][1] = 0;
+        const int64_t l1 = lptr[it + 1];
+        for (int64_t l = lptr[it] + tm.base;; l += Tm::PER_WARP * Tm::LANES) {
+            const int n = tm.on && l < l1 ? (int)(l1 - l < Tm::LANES ? l1 - l : Tm::LANES) : 0;
+            const int nmax = __reduce_max_sync(0xffffffffu, n);
+            if (nmax == 0) break;
+            int32_t ia = 0, ib = 0;
+            if (tm.e < n) {
+                ia = la[l + tm.e];
+                ib = lb[l + tm.e];
+            }
+            for (int j = 0; j < nmax; j += U) {
+                V2 p[U][BC / 2], ap[U];
+                int32_t xa[U], xb[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int src = tm.base + j + u < 32 ? tm.base + j + u : 31;
+                    xa[u] = __shfl_sync(0xffffffffu, ia, src);
+                    xb[u] = __shfl_sync(0xffffffffu, ib, src);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int64_t ka = xa[u], kb = xb[u];
+                    ap[u].x = ap[u].y = 0;
+#pragma unroll
+                    for (int r = 0; r < BC / 2; ++r) p[u][r].x = p[u][r].y = 0;
+                    if (j + u < n) {
+                        ap[u] = __ldg(reinterpret_cast<const V2 *>(AP + kb * B * BC) + tm.e);
+                        const V2 *pr = reinterpret_cast<const V2 *>(P + ka * B * BC) + tm.m * (BC / 2);
+#pragma unroll
+                        for (int r = 0; r < BC / 2; ++r) p[u][r] = __ldg(pr + r);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int r = 0; r < BC / 2; ++r) {
+                        acc[2 * r][0] += (T)p[u][r].x * (T)ap[u].x;
+                        acc[2 * r][1] += (T)p[u][r].x * (T)ap[u].y;
+                        acc[2 * r + 1][0] += (T)p[u][r].y * (T)ap[u].x;
+                        acc[2 * r + 1][1] += (T)p[u][r].y * (T)ap[u].y;
+                    }
+            }
+        }
+        T out[BC / B][2];
+        tm.template reduce<BC, T>(acc, out);
+        tm.join(out);
+        if (tm.on && tm.team == 0) {
+            const int64_t q = qmap ? (int64_t)qmap[it] : it;
+            const int64_t I = row[q], J = col[q];
+#pragma unroll
+            for (int t = 0; t < BC / B; ++t) {
+                const int r = t * B + tm.m;
+                V w[2];
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    const int c = 2 * tm.h + s;
+                    w[s] = (V)out[t][s];
+                    if (dead[I * BC + r] || dead[J * BC + c]) w[s] = (I == J && r == c) ? (V)1 : (V)0;
+                }
+                V2 o;
+                o.x = w[0];
+                o.y = w[1];
+                reinterpret_cast<V2 *>(Ac + q * BC * BC + r * BC)[tm.h] = o;
+            }
+        }
+    }
+}
+
 // lanes per output block for the lane-group gathers: about 8 or more pairs per lane
 inline int gather_lanes(int64_t nblk, int64_t pairs) {
     const double avg = nblk > 0 ? (double)pairs / (double)nblk : 0.0;
@@ -754,6 +1003,51 @@ static void gather_Ac_groups(int64_t nitems, int64_t pairs, const int32_t *qmap,
     }
 }
 
+// One thread per output block, or a group of lanes per block where blocks are few or each sums
+// many pairs (the small coarse levels 10-20x faster).  For 3 x 6 blocks teams replace the thread
+// per block of A P and the groups of eight of P'(A P): those sum chains of the same length or
+// shorter, so the FP32 form rounds no more than it did; longer lists stay with larger groups.
+// (6 x 6 blocks would take 18 lanes, one team a warp: A P of the layered slope's second level
+// 1.36 against 0.53 ms with lane groups.)
+template <int B, int BC> constexpr bool by_teams() { return B == 3 && BC == 6; }
+inline bool by_groups(int64_t nblk, int64_t pairs) { return nblk < 32768 || pairs >= 24 * nblk; }
+
+template <int B, int BC, typename V>
+static void gather_AP(const Level &L, const V *A, const V *P, V *AP, cudaStream_t st) {
+    const int64_t nblk = L.AP.nblk, *ptr = L.ap_plan.d_ptr;
+    const int32_t *la = L.ap_plan.d_a, *lb = L.ap_plan.d_b;
+    if (by_groups(nblk, L.ap_pairs)) {
+        gather_AP_groups<B, BC, V>(nblk, L.ap_pairs, ptr, la, lb, A, P, AP, st);
+    } else if constexpr (by_teams<B, BC>()) {
+        k_team_AP<B, BC, V><<<grid_chunks(nblk, TP_RUN), 128, 0, st>>>(nblk, L.AP.d_row, L.d_Arp, ptr, la, lb, A, P, AP);
+    } else {
+        const int64_t ch = chunk_len(nblk, 128, 8 * 128);
+        k_gather_AP<B, BC, V><<<grid_chunks(nblk, ch), 128, 0, st>>>(nblk, ptr, la, lb, A, P, AP, ch);
+    }
+}
+
+template <int B, int BC, typename V>
+static void gather_Ac(int64_t nitems, int64_t pairs, const int32_t *qmap, const int32_t *row, const int32_t *col,
+                      const int64_t *ptr, const int32_t *la, const int32_t *lb, const V *P, const V *AP,
+                      const uint8_t *dead, V *Ac, cudaStream_t st) {
+    if constexpr (by_teams<B, BC>()) {
+        if (gather_lanes(nitems, pairs) == 8) {
+            // a block per warp in FP64 (0.73 ms against 0.96 with runs of 32), runs in FP32 (1.52 ms against 1.70)
+            const int64_t ch = chunk_len(nitems, 4, sizeof(V) == 8 ? 4 : 32);
+            k_team_Ac<B, BC, V><<<grid_chunks(nitems, ch), 128, 0, st>>>(nitems, qmap, row, col, ptr, la, lb, P, AP, dead, Ac,
+                                                                         ch);
+            return;
+        }
+    }
+    if (by_groups(nitems, pairs)) {
+        gather_Ac_groups<B, BC, V>(nitems, pairs, qmap, row, col, ptr, la, lb, P, AP, dead, Ac, st);
+    } else {
+        const int64_t ch = chunk_len(nitems, 128, 8 * 128);
+        k_gather_Ac<B, BC, V><<<grid_chunks(nitems, ch), 128, 0, st>>>(nitems, qmap, row, col, ptr, la, lb, P, AP, dead, Ac,
+                                                                       ch);
+    }
+}
+
 // Blocks below the diagonal of a symmetric Galerkin matrix: A(dst) = A(src)'.  A thread per
 // entry, so the writes of a block are one run and its reads stay within one block (a thread per
 // block strode BC * BC values between lanes: 123 against 28 us a level on the layered slope).
@@ -775,17 +1069,8 @@ static void galerkin_Ac(const Level &L, const Level &C, const V *P, const V *AP,
     const bool sym = L.d_ac_out != nullptr;
     const int64_t items = sym ? L.n_ac_items : C.Anblk;
     const int32_t *qmap = sym ? L.d_ac_out : nullptr;
-    // one thread per output block, or a group of lanes per block where blocks are few or
-    // each sums many pairs (on the SSR hierarchy: fine-level P'(A P), ~63 pairs per block,
-    // 1.3x faster per lane group; the small coarse levels 10-20x faster)
-    if (!(items < 32768 || L.ac_pairs >= 24 * items)) {
-        const int64_t ch = chunk_len(items, 128, 8 * 128);
-        k_gather_Ac<B, BC, V><<<grid_chunks(items, ch), 128, 0, st>>>(items, qmap, C.Aown.d_row, C.d_Acol,
-                                                                      L.ac_plan.d_ptr, L.ac_plan.d_a, L.ac_plan.d_b,
-                                                                      P, AP, C.d_dead, Ac, ch);
-    } else
-        gather_Ac_groups<B, BC, V>(items, L.ac_pairs, qmap, C.Aown.d_row, C.d_Acol, L.ac_plan.d_ptr, L.ac_plan.d_a,
-                                   L.ac_plan.d_b, P, AP, C.d_dead, Ac, st);
+    gather_Ac<B, BC, V>(items, L.ac_pairs, qmap, C.Aown.d_row, C.d_Acol, L.ac_plan.d_ptr, L.ac_plan.d_a, L.ac_plan.d_b, P,
+                        AP, C.d_dead, Ac, st);
     if (sym && L.n_ac_lower > 0)
         k_mirror_blocks<BC, V><<<grid_for(L.n_ac_lower * BC * BC, 256, 16), 256, 0, st>>>(L.n_ac_lower, L.d_ac_lower,
                                                                            L.d_ac_lower_src, Ac);
@@ -1279,19 +1564,7 @@ static int numeric_transfer(sg_amg *h, int l, cudaStream_t st) {
             L.P.nblk, L.P.d_row, L.P.d_col, L.at_plan.d_ptr, L.at_plan.d_a, L.d_Acol, A, L.T, L.d_agg, L.Dinv, L.lmax,
             h->opt.omega_scale, L.Pv, pch);
         k_transpose_blocks<BB, BC><<<grid_for(L.P.nblk * BB * BC, 256), 256, 0, st>>>(L.P.nblk, L.d_R_from_P, L.Pv, L.Rv);
-        // one thread per output block, or a warp per block where blocks are few or each sums
-        // many pairs (measured on the SSR hierarchy: fine-level A P, ~15 pairs per block, is
-        // faster per thread; P'(A P), ~63 pairs per block, 1.3x faster per warp; the small
-        // coarse levels 10-20x faster per warp)
-        auto per_warp = [](int64_t nblk, int64_t pairs) { return nblk < 32768 || pairs >= 24 * nblk; };
-        if (!per_warp(L.AP.nblk, L.ap_pairs)) {
-            const int64_t ach = chunk_len(L.AP.nblk, 128, 8 * 128);
-            k_gather_AP<BB, BC><<<grid_chunks(L.AP.nblk, ach), 128, 0, st>>>(L.AP.nblk, L.ap_plan.d_ptr,
-                                                                             L.ap_plan.d_a, L.ap_plan.d_b, A, L.Pv,
-                                                                             L.APv, ach);
-        } else
-            gather_AP_groups<BB, BC, double>(L.AP.nblk, L.ap_pairs, L.ap_plan.d_ptr, L.ap_plan.d_a, L.ap_plan.d_b, A,
-                                             L.Pv, L.APv, st);
+        gather_AP<BB, BC, double>(L, A, L.Pv, L.APv, st);
         galerkin_Ac<BB, BC, double>(L, C, L.Pv, L.APv, C.Aown_vals, st);
     }));
     SG_CUDA(cudaGetLastError());
@@ -1391,14 +1664,7 @@ static int numeric_update32(sg_amg *h, cudaStream_t st) {
                 L.Dinv, L.lmax, h->opt.omega_scale, L.P32, pch);
             k_transpose_blocks<BB, BC, float><<<grid_for(L.P.nblk * BB * BC, 256), 256, 0, st>>>(
                 L.P.nblk, L.d_R_from_P, L.P32, L.R32);
-            auto per_warp = [](int64_t nblk, int64_t pairs) { return nblk < 32768 || pairs >= 24 * nblk; };
-            if (!per_warp(L.AP.nblk, L.ap_pairs)) {
-                const int64_t ach = chunk_len(L.AP.nblk, 128, 8 * 128);
-                k_gather_AP<BB, BC, float><<<grid_chunks(L.AP.nblk, ach), 128, 0, st>>>(
-                    L.AP.nblk, L.ap_plan.d_ptr, L.ap_plan.d_a, L.ap_plan.d_b, L.A32, L.P32, L.APv32, ach);
-            } else
-                gather_AP_groups<BB, BC, float>(L.AP.nblk, L.ap_pairs, L.ap_plan.d_ptr, L.ap_plan.d_a, L.ap_plan.d_b,
-                                                L.A32, L.P32, L.APv32, st);
+            gather_AP<BB, BC, float>(L, L.A32, L.P32, L.APv32, st);
             galerkin_Ac<BB, BC, float>(L, C, L.P32, L.APv32, C.A32, st);
         }));
         SG_CUDA(cudaGetLastError());
