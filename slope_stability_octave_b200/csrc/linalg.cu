@@ -62,6 +62,12 @@ struct ChebRow {
 
 // rows of a CTA of k_spmv_blk: four per warp slot
 #define SPMV_MAX_ROWS(G) (32 * (32 / (G)))
+// Entries a lane of a scalar matrix loads before its products.  Rows of 28 entries (seepage, P2
+// tetrahedra, 60k rows, in L2) with one entry per lane of a warp wait on one chain col -> x per row and shuffle
+// five times: 7.7 us; sixteen lanes with two entries each 7.1 us, with the Chebyshev step 7.2 -> 6.1 us
+// (eight lanes with four entries: the same).
+constexpr int SPMV_SCALAR_LOADS = 2;
+
 template <int BR, int BC, int G, typename VT, typename XT, bool CHEB = false>
 __global__ void __launch_bounds__(256) k_spmv_blk(int64_t nrows, const int32_t *__restrict__ rp,
                                                   const int32_t *__restrict__ col, const VT *__restrict__ vals,
@@ -87,16 +93,33 @@ __global__ void __launch_bounds__(256) k_spmv_blk(int64_t nrows, const int32_t *
         for (int a = 0; a < BR; ++a) acc[a] = 0;
         if (row < rend) {
             const int32_t p1 = rp[row + 1];
-            for (int32_t p = rp[row] + gl; p < p1; p += G) {
-                const int64_t j = col[p];
-                A xj[BC];
+            if constexpr (BR * BC == 1) {
+                for (int32_t p = rp[row] + gl; p < p1; p += G * SPMV_SCALAR_LOADS) {
+                    int32_t j[SPMV_SCALAR_LOADS];
+                    A v[SPMV_SCALAR_LOADS], xj[SPMV_SCALAR_LOADS];
 #pragma unroll
-                for (int b = 0; b < BC; ++b) xj[b] = (A)x[j * BC + b];
-                const VT *v = vals + (int64_t)p * BR * BC;
+                    for (int u = 0; u < SPMV_SCALAR_LOADS; ++u) {
+                        const int32_t q = p + u * G;
+                        j[u] = q < p1 ? col[q] : -1;
+                        v[u] = q < p1 ? (A)vals[q] : (A)0;
+                    }
 #pragma unroll
-                for (int a = 0; a < BR; ++a)
+                    for (int u = 0; u < SPMV_SCALAR_LOADS; ++u) xj[u] = j[u] >= 0 ? (A)x[j[u]] : (A)0;
 #pragma unroll
-                    for (int b = 0; b < BC; ++b) acc[a] += (A)v[a * BC + b] * xj[b];
+                    for (int u = 0; u < SPMV_SCALAR_LOADS; ++u) acc[0] += v[u] * xj[u];
+                }
+            } else {
+                for (int32_t p = rp[row] + gl; p < p1; p += G) {
+                    const int64_t j = col[p];
+                    A xj[BC];
+#pragma unroll
+                    for (int b = 0; b < BC; ++b) xj[b] = (A)x[j * BC + b];
+                    const VT *v = vals + (int64_t)p * BR * BC;
+#pragma unroll
+                    for (int a = 0; a < BR; ++a)
+#pragma unroll
+                        for (int b = 0; b < BC; ++b) acc[a] += (A)v[a * BC + b] * xj[b];
+                }
             }
         }
 #pragma unroll
@@ -297,7 +320,7 @@ static void spmv_launch(int64_t nrows, int64_t nblk, const int32_t *rp, const in
             k_spmv_row<BR, BC, 16, 2, VT, XT, CHEB><<<grid, 256, 0, st>>>(nrows, rp, col, vals, x, y, alpha, beta, bvec, mode, cheb);
         }
     } else {
-        const int G = avg >= 16.0 ? 32 : (avg >= 8.0 ? 16 : 8);
+        const int G = BR * BC == 1 ? (avg >= 12.0 ? 16 : 8) : avg >= 16.0 ? 32 : (avg >= 8.0 ? 16 : 8);
         // up to four rows (G = 32) or 16 rows (G = 8) per warp
         const int64_t rpc = chunk_len(nrows, 8 * (32 / G), SPMV_MAX_ROWS(G));
         const unsigned grid = grid_chunks(nrows, rpc);
