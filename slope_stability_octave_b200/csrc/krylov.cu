@@ -54,6 +54,7 @@ struct sg_krylov {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
     uint64_t gkey = 0;
+    bool gproj = false;         // the captured loop forms A z for the projection
     int64_t launches_start = 0, launches_body = 0, launches_end = 0;
     int use_graph = 1;
     // blocked A-orthogonalisation: A times the block's input columns (n x 16), the block's
@@ -126,19 +127,17 @@ __global__ void k_anorm_scale(int64_t n, const double *__restrict__ ntp, double 
 
 // ------------------------------------------------------------------ graph-replayed solve
 
-// the basis column j (j read from the device) into w, and back
-__global__ void k_col_get(int64_t n, const double *__restrict__ V, const int32_t *__restrict__ j,
-                          double *__restrict__ w) {
-    const double *c = V + (int64_t)j[0] * n;
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
-        w[r] = c[r];
-}
-__global__ void k_col_put(int64_t n, const double *__restrict__ w, double *__restrict__ V,
-                          const int32_t *__restrict__ j, const double *__restrict__ scale) {
+// The next basis vector, scale[0] w, into column j of V (j read from the device) and into
+// next, from where the next iteration reads it (w may be that column).
+__global__ void k_col_put(int64_t n, const double *w, double *V, const int32_t *__restrict__ j,
+                          const double *__restrict__ scale, double *__restrict__ next) {
     double *c = V + (int64_t)j[0] * n;
-    const double s = scale ? scale[0] : 1.0;
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
-        c[r] = scale ? w[r] * s : w[r];
+    const double s = scale[0];
+    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
+        const double v = w[r] * s;
+        c[r] = v;
+        next[r] = v;
+    }
 }
 
 __global__ void k_fg_params(int32_t *st, double *sc, const double **ptrs, double tol, int maxit, int k,
@@ -174,21 +173,40 @@ __global__ void k_fg_start(cudaGraphConditionalHandle h, int mcap, int32_t *st, 
 // End of iteration j: the new Hessenberg column (the two CGS passes' coefficients), the
 // previous Givens rotations and a new one, the residual estimate |g_{j+1}| / |b|, the scale of
 // the next basis vector and the loop condition -- the host loop's arithmetic, on the device.
-__global__ void k_fg_arnoldi(cudaGraphConditionalHandle h, int mcap, int32_t *st, double *sc,
-                             const double *__restrict__ h1, const double *__restrict__ h2,
-                             const double *__restrict__ hn, double *H, double *cs, double *sn, double *g,
-                             double *hist) {
-    if (threadIdx.x != 0) return;
+// One warp: the previous rotations are a serial chain, so their inputs are fetched 32 at a time
+// into shared memory and the carried entry stays in a register.  hn: DOT_BLOCKS partial sums of the new vector's squared norm.
+__global__ void __launch_bounds__(32) k_fg_arnoldi(cudaGraphConditionalHandle h, int mcap, int32_t *st, double *sc,
+                                                   const double *__restrict__ h1, const double *__restrict__ h2,
+                                                   const double *__restrict__ hn, double *H, double *cs, double *sn,
+                                                   double *g, double *hist) {
+    __shared__ double sh[32], sco[32], ssi[32], so[32];
+    const int lane = threadIdx.x;
     const int j = st[0];
-    for (int i = 0; i <= j; ++i) H[(size_t)i * mcap + j] = h1[i] + h2[i];
-    const double hjj = sqrt(hn[0]);
-    H[(size_t)(j + 1) * mcap + j] = hjj;
-    for (int i = 0; i < j; ++i) {
-        const double a = H[(size_t)i * mcap + j], bb = H[(size_t)(i + 1) * mcap + j];
-        H[(size_t)i * mcap + j] = cs[i] * a + sn[i] * bb;
-        H[(size_t)(i + 1) * mcap + j] = -sn[i] * a + cs[i] * bb;
+    double nn = 0.0;
+    for (int i = lane; i < DOT_BLOCKS; i += 32) nn += hn[i];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) nn += __shfl_xor_sync(0xffffffffu, nn, off);
+    double a = h1[0] + h2[0];
+    for (int i0 = 0; i0 < j; i0 += 32) {
+        const int i = i0 + lane;
+        if (i < j) {
+            sh[lane] = h1[i + 1] + h2[i + 1];
+            sco[lane] = cs[i];
+            ssi[lane] = sn[i];
+        }
+        __syncwarp();
+        if (lane == 0)
+            for (int t = 0; t < 32 && i0 + t < j; ++t) {
+                const double b = sh[t], c = sco[t], s = ssi[t];
+                so[t] = c * a + s * b;
+                a = -s * a + c * b;
+            }
+        __syncwarp();
+        if (i < j) H[(size_t)i * mcap + j] = so[lane];
+        __syncwarp();
     }
-    const double a = H[(size_t)j * mcap + j], bb = H[(size_t)(j + 1) * mcap + j];
+    if (lane != 0) return;
+    const double hjj = sqrt(nn), bb = hjj;
     const double den = hypot(a, bb);
     cs[j] = den > 0 ? a / den : 1.0;
     sn[j] = den > 0 ? bb / den : 0.0;
@@ -206,14 +224,34 @@ __global__ void k_fg_arnoldi(cudaGraphConditionalHandle h, int mcap, int32_t *st
     cudaGraphSetConditional(h, go ? 1u : 0u);
 }
 
-// y = R \ g over the iterations done
-__global__ void k_fg_solve_y(int mcap, const int32_t *st, const double *H, const double *g, double *y) {
-    if (threadIdx.x != 0) return;
+// y = R \ g over the iterations done: the triangle in shared memory up to 64 iterations, a warp
+// per row's sum (one thread reading H in memory took 42 us at 30 iterations).
+constexpr int FG_TRI = 64;
+__global__ void __launch_bounds__(256) k_fg_solve_y(int mcap, const int32_t *st, const double *__restrict__ H,
+                                                    const double *__restrict__ g, double *y) {
+    __shared__ double tri[FG_TRI * FG_TRI];
     const int it = st[0];
+    const bool small = it <= FG_TRI;
+    if (small)
+        for (int t = threadIdx.x; t < it * it; t += blockDim.x) {
+            const int i = t / it, c = t - i * it;
+            if (c >= i) tri[i * FG_TRI + c] = H[(size_t)i * mcap + c];
+        }
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
+    const double *R = small ? tri : H;
+    const size_t ld = small ? FG_TRI : mcap;
     for (int i = it - 1; i >= 0; --i) {
-        double s = g[i];
-        for (int c = i + 1; c < it; ++c) s -= H[(size_t)i * mcap + c] * y[c];
-        y[i] = H[(size_t)i * mcap + i] != 0.0 ? s / H[(size_t)i * mcap + i] : 0.0;
+        double s = 0.0;
+        for (int c = i + 1 + lane; c < it; c += 32) s += R[i * ld + c] * y[c];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+        if (lane == 0) {
+            const double d = R[i * ld + i];
+            y[i] = d != 0.0 ? (g[i] - s) / d : 0.0;
+        }
+        __syncwarp();
     }
 }
 
@@ -245,13 +283,14 @@ static void graph_release(sg_krylov *ws) {
     ws->gkey = 0;
 }
 
-// Captures start, loop and least-squares solve for (A, Avals, M) into ws->gexec.
-static int graph_capture(sg_krylov *ws, const sg_bsr *A, const double *Avals, sg_amg *M) {
+// Captures start, loop and least-squares solve for (A, Avals, M) into ws->gexec.  form_az: the
+// projection z - W W'(A z) with A z formed by an SpMV (A W is not given: A is not symmetric).
+static int graph_capture(sg_krylov *ws, const sg_bsr *A, const double *Avals, sg_amg *M, bool form_az) {
     graph_release(ws);
     const int64_t n = ws->n;
     const int m = ws->maxit;
     const int kcap = (int)ws->kcap;
-    double *h1 = ws->hdev, *h2 = ws->hdev + (m + 2), *hn = ws->hdev + 2 * (m + 2);
+    double *h1 = ws->hdev, *h2 = ws->hdev + (m + 2);
     InstrSuspend quiet;   // no event records inside the graph
     int rc = SG_OK;
     cudaStream_t cap = ws->cap, cap2 = ws->cap2;
@@ -275,8 +314,8 @@ static int graph_capture(sg_krylov *ws, const sg_bsr *A, const double *Avals, sg
     const int64_t l0 = sg_launch_count(0);
     count_launch(1);
     k_fg_start<<<1, 32, 0, cap>>>(hcond, m, ws->dstate, ws->dscal, ws->dg, ws->dhist);
-    if (scale_dev(n, ws->V, ws->dscal + 3, 0, ws->V, cap) || cudaGetLastError() != cudaSuccess)
-        return abort_capture(set_error(SG_ERR_CUDA, "capture start"));
+    k_col_put<<<grid_for(n, 256, 8), 256, 0, cap>>>(n, ws->V, ws->V, ws->dstate, ws->dscal + 3, ws->w);
+    if (cudaGetLastError() != cudaSuccess) return abort_capture(set_error(SG_ERR_CUDA, "capture start"));
     const int64_t l1 = sg_launch_count(0);
     if (cudaStreamGetCaptureInfo(cap, &status, nullptr, &g, &deps, &ndeps) != cudaSuccess)
         return abort_capture(set_error(SG_ERR_CUDA, "capture info"));
@@ -295,24 +334,26 @@ static int graph_capture(sg_krylov *ws, const sg_bsr *A, const double *Avals, sg
     if (cudaStreamBeginCaptureToGraph(cap2, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
         return abort_capture(set_error(SG_ERR_CUDA, "body capture"));
     {
-        k_col_get<<<grid_for(n, 256, 8), 256, 0, cap2>>>(n, ws->V, ws->dstate, ws->w);
         if (M) rc = sg_amg_apply(M, ws->w, ws->t, cap2);
         else if (cudaMemcpyAsync(ws->t, ws->w, sizeof(double) * n, cudaMemcpyDeviceToDevice, cap2) != cudaSuccess)
             rc = set_error(SG_ERR_CUDA, "body copy");
-        if (!rc) rc = multidot_dc(n, ws->dstate + 1, 0, kcap, nullptr, ws->dptr + 1, n, ws->t, ws->part, ws->hd, cap2);
-        if (!rc) rc = gemv_dc(-1, n, ws->dstate + 1, 0, kcap, nullptr, ws->dptr, n, ws->hd, ws->t, cap2);
-        if (!rc) k_col_put<<<grid_for(n, 256, 8), 256, 0, cap2>>>(n, ws->t, ws->Z, ws->dstate, nullptr);
+        if (form_az) {
+            if (!rc) rc = bsr_spmv<double, double>(*A, Avals, ws->t, ws->u, 1.0, 0.0, cap2);
+            if (!rc) rc = multidot_dc(n, ws->dstate + 1, 0, kcap, nullptr, ws->dptr, n, ws->u, ws->part, ws->hd, cap2);
+        } else if (!rc) {
+            rc = multidot_dc(n, ws->dstate + 1, 0, kcap, nullptr, ws->dptr + 1, n, ws->t, ws->part, ws->hd, cap2);
+        }
+        if (!rc) rc = gemv_dc(-1, n, ws->dstate + 1, 0, kcap, nullptr, ws->dptr, n, ws->hd, ws->t, cap2, ws->Z, ws->dstate);
         if (!rc) rc = bsr_spmv<double, double>(*A, Avals, ws->t, ws->u, 1.0, 0.0, cap2);
         if (!rc) rc = multidot_dc(n, ws->dstate, 1, m, ws->V, nullptr, n, ws->u, ws->part, h1, cap2);
         if (!rc) rc = gemv_dc(-1, n, ws->dstate, 1, m, ws->V, nullptr, n, h1, ws->u, cap2);
         if (!rc) rc = multidot_dc(n, ws->dstate, 1, m, ws->V, nullptr, n, ws->u, ws->part, h2, cap2);
-        if (!rc) rc = gemv_dc(-1, n, ws->dstate, 1, m, ws->V, nullptr, n, h2, ws->u, cap2);
-        if (!rc) rc = multidot(n, 1, ws->u, n, ws->u, ws->part, hn, cap2);
+        if (!rc) rc = gemv_dc(-1, n, ws->dstate, 1, m, ws->V, nullptr, n, h2, ws->u, cap2, nullptr, nullptr, ws->part);
         if (!rc) {
             count_launch(1);
-            k_fg_arnoldi<<<1, 32, 0, cap2>>>(hcond, m, ws->dstate, ws->dscal, h1, h2, hn, ws->dH, ws->dcs, ws->dsn,
+            k_fg_arnoldi<<<1, 32, 0, cap2>>>(hcond, m, ws->dstate, ws->dscal, h1, h2, ws->part, ws->dH, ws->dcs, ws->dsn,
                                              ws->dg, ws->dhist);
-            k_col_put<<<grid_for(n, 256, 8), 256, 0, cap2>>>(n, ws->u, ws->V, ws->dstate, ws->dscal + 3);
+            k_col_put<<<grid_for(n, 256, 8), 256, 0, cap2>>>(n, ws->u, ws->V, ws->dstate, ws->dscal + 3, ws->w);
         }
         cudaGraph_t body_out = nullptr;
         const cudaError_t e = cudaStreamEndCapture(cap2, &body_out);
@@ -321,7 +362,7 @@ static int graph_capture(sg_krylov *ws, const sg_bsr *A, const double *Avals, sg
     if (rc) return abort_capture(rc);
     const int64_t l2 = sg_launch_count(0);
     count_launch(1);
-    k_fg_solve_y<<<1, 32, 0, cap>>>(m, ws->dstate, ws->dH, ws->dg, ws->dy);
+    k_fg_solve_y<<<1, 256, 0, cap>>>(m, ws->dstate, ws->dH, ws->dg, ws->dy);
     cudaGraph_t full = nullptr;
     if (cudaStreamEndCapture(cap, &full) != cudaSuccess || !full) {
         if (full) cudaGraphDestroy(full);
@@ -362,10 +403,12 @@ static int dfgmres_graph(sg_krylov *ws, const sg_bsr *A, const double *Avals, sg
     int rc = graph_alloc(ws);
     if (rc) return rc;
     const uint64_t key = graph_key(ws, A, Avals, M);
-    if (!ws->gexec || ws->gkey != key) {
-        rc = graph_capture(ws, A, Avals, M);
+    const bool form_az = k > 0 && !AWd;
+    if (!ws->gexec || ws->gkey != key || (k > 0 && ws->gproj != form_az)) {
+        rc = graph_capture(ws, A, Avals, M, form_az);
         if (rc) return rc;
         ws->gkey = key;
+        ws->gproj = form_az;
     }
     // x0 = Wd (Wd' b), r0 = b - A x0 = V(:, 0), b'b and r0'r0, the solve's parameters
     SG_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * n, st));
@@ -477,7 +520,7 @@ extern "C" int sg_dfgmres_solve(sg_krylov *ws, const sg_bsr *A, const double *Av
     const cudaStream_t st = as_stream(stream);
     int rc = ensure_kcap(ws, std::max<int64_t>(k, 1));
     if (rc) return rc;
-    if (ws->use_graph && (k == 0 || AWd))
+    if (ws->use_graph)
         return dfgmres_graph(ws, A, Avals, M, Wd, AWd, k, b, x, tol, maxit, iters, relres, res_hist, st);
     double *part = ws->part, *hdev = ws->hdev, *hp = ws->hpin;
     const unsigned gb = grid_for(n, 256, 8);

@@ -1584,20 +1584,34 @@ __global__ void k_reduce_partials_dc(const int32_t *__restrict__ cnt, int add, i
     }
 }
 
+// copy: the result also goes to column copy_col[0] of copy (leading dimension n).  sq: w'w of the result,
+// one partial sum per CTA.  Both save a pass and a launch after the product (an iteration of the
+// replayed loop on vectors that fit L2 is a row of 2 us launches).
 template <int SIGN>
-__global__ void k_gemv_dc(int64_t n, const int32_t *__restrict__ cnt, int add, int mmax, const double *V,
-                          const double *const *Vp, int64_t ldv, const double *__restrict__ h,
-                          double *__restrict__ w) {
+__global__ void __launch_bounds__(256) k_gemv_dc(int64_t n, const int32_t *__restrict__ cnt, int add, int mmax,
+                                                 const double *V, const double *const *Vp, int64_t ldv,
+                                                 const double *__restrict__ h, double *__restrict__ w, double *copy,
+                                                 const int32_t *__restrict__ copy_col, double *__restrict__ sq) {
     extern __shared__ double hs[];
-    const int m = min(cnt[0] + add, mmax);
+    __shared__ double sh[32];
+    const int m = max(0, min(cnt[0] + add, mmax));
     const double *__restrict__ B = V ? V : Vp[0];
     for (int i = threadIdx.x; i < m; i += blockDim.x) hs[i] = h[i];
     __syncthreads();
-    if (m <= 0) return;
+    if (m == 0 && !copy && !sq) return;
+    double *__restrict__ c = copy ? copy + (int64_t)copy_col[0] * n : nullptr;
+    double ss = 0;
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
         double s = 0;
         for (int i = 0; i < m; ++i) s += hs[i] * B[i * ldv + r];
-        w[r] = SIGN > 0 ? w[r] + s : w[r] - s;
+        const double v = SIGN > 0 ? w[r] + s : w[r] - s;
+        if (m > 0) w[r] = v;
+        if (c) c[r] = v;
+        ss += v * v;
+    }
+    if (sq) {
+        ss = block_sum(ss, sh);
+        if (threadIdx.x == 0) sq[blockIdx.x] = ss;
     }
 }
 
@@ -1612,11 +1626,12 @@ int multidot_dc(int64_t n, const int32_t *cnt, int add, int mmax, const double *
 }
 
 int gemv_dc(int sign, int64_t n, const int32_t *cnt, int add, int mmax, const double *V, const double *const *Vp,
-            int64_t ldv, const double *h, double *w, cudaStream_t st) {
-    if (mmax <= 0) return SG_OK;
-    const unsigned grid = grid_for(n, 256, 8);
-    if (sign > 0) k_gemv_dc<1><<<grid, 256, sizeof(double) * mmax, st>>>(n, cnt, add, mmax, V, Vp, ldv, h, w);
-    else k_gemv_dc<-1><<<grid, 256, sizeof(double) * mmax, st>>>(n, cnt, add, mmax, V, Vp, ldv, h, w);
+            int64_t ldv, const double *h, double *w, cudaStream_t st, double *copy, const int32_t *copy_col, double *sq) {
+    if (mmax <= 0 && !copy && !sq) return SG_OK;
+    count_launch(sq ? 1 : 0);
+    const unsigned grid = sq ? DOT_BLOCKS : grid_for(n, 256, 8);
+    if (sign > 0) k_gemv_dc<1><<<grid, 256, sizeof(double) * mmax, st>>>(n, cnt, add, mmax, V, Vp, ldv, h, w, copy, copy_col, sq);
+    else k_gemv_dc<-1><<<grid, 256, sizeof(double) * mmax, st>>>(n, cnt, add, mmax, V, Vp, ldv, h, w, copy, copy_col, sq);
     SG_CUDA(cudaGetLastError());
     return SG_OK;
 }
@@ -1628,20 +1643,6 @@ __global__ void k_axpby(int64_t n, double a, const double *__restrict__ x, doubl
 
 int axpby(int64_t n, double a, const double *x, double b, double *y, cudaStream_t st) {
     k_axpby<<<grid_for(n, 256, 8), 256, 0, st>>>(n, a, x, b, y);
-    SG_CUDA(cudaGetLastError());
-    return SG_OK;
-}
-
-// y = x * s, s = num[0] (invert: 1 / num[0])
-__global__ void k_scale(int64_t n, const double *__restrict__ x, const double *__restrict__ num, int invert,
-                        double *__restrict__ y) {
-    const double s = invert ? 1.0 / num[0] : num[0];
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
-        y[r] = x[r] * s;
-}
-
-int scale_dev(int64_t n, const double *x, const double *num, int invert, double *y, cudaStream_t st) {
-    k_scale<<<grid_for(n, 256, 8), 256, 0, st>>>(n, x, num, invert, y);
     SG_CUDA(cudaGetLastError());
     return SG_OK;
 }

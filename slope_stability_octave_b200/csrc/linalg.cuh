@@ -105,13 +105,13 @@ int ts_apply_pair(int64_t n, int k, const int32_t *kout, const int32_t *pmap, co
 // V, or *Vp when V is null (both on the device)
 int multidot_dc(int64_t n, const int32_t *cnt, int add, int mmax, const double *V, const double *const *Vp,
                 int64_t ldv, const double *w, double *partial, double *out, cudaStream_t st);
-// w += sign * V(:, 0:m) h
+// w += sign * V(:, 0:m) h; also into column copy_col[0] of copy (n rows) if given, and, if sq is given,
+// DOT_BLOCKS partial sums of w'w
 int gemv_dc(int sign, int64_t n, const int32_t *cnt, int add, int mmax, const double *V, const double *const *Vp,
-            int64_t ldv, const double *h, double *w, cudaStream_t st);
+            int64_t ldv, const double *h, double *w, cudaStream_t st, double *copy = nullptr,
+            const int32_t *copy_col = nullptr, double *sq = nullptr);
 
 // y = a x + b y
 int axpby(int64_t n, double a, const double *x, double b, double *y, cudaStream_t st);
-// y = x * s where s = *num / *den on the device (den may be null -> s = *num)
-int scale_dev(int64_t n, const double *x, const double *num, int invert, double *y, cudaStream_t st);
 
 }  // namespace sg
