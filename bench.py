@@ -654,7 +654,7 @@ def run_box(args, rank):
     e2e_ms = (time.perf_counter() - t0) * 1e3 / args.steps + t_asm
     peak, peak_kind = peaks()
     b_sds = n * 416
-    b_asm = dm.n_e * 5896 + dm.n_blocks * 72
+    b_asm = dm.n_e * 4048 + dm.n_blocks * 72
     ach_sds = b_sds / (t_sds * 1e-3) / 1e9
     ach_asm = b_asm / (t_asm * 1e-3) / 1e9
     cpu = None
@@ -671,9 +671,9 @@ def run_box(args, rank):
                           "-O2 -fopenmp, best of 3")
     rows = {"return_map": dict(kernel="k_mc3d<S and DS>", ms=t_sds, algorithmic_bytes=b_sds, achieved=ach_sds,
                                frac=ach_sds / peak),
-            "assembly": dict(kernel="k_element_blocks_p2tet + k_gather_blocks3 (deterministic B'DB)", ms=t_asm,
+            "assembly": dict(kernel="k_element_blocks_fact + k_gather_upper (deterministic B'DB)", ms=t_asm,
                              algorithmic_bytes=b_asm, achieved=ach_asm, frac=ach_asm / peak,
-                             fp64_tflops=dm.n_e * 71280 / (t_asm * 1e-3) / 1e12)}
+                             fp64_tflops=dm.n_e * 28000 / (t_asm * 1e-3) / 1e12)}
     top = max(rows, key=lambda k: rows[k]["ms"])
     r = rows[top]
     line = dict(metric=BOX_METRIC, value=ms, unit="ms/pass", n_gpus=args.gpus, steps=args.steps,
@@ -721,24 +721,26 @@ KINDS = ["spmv3_f64", "spmv3_f32", "constitutive_S_DS", "constitutive_S", "assem
 KIND_NAMES = {
     "spmv3_f64": "k_spmv_blk 3x3 FP64, fine level (Arnoldi, projection, residuals)",
     "spmv3_f32": "k_spmv_blk 3x3 FP32, fine level of the FP32 V-cycle",
-    "constitutive_S_DS": "k_mc3d return mapping + tangent",
+    "constitutive_S_DS": "k_response3d<tangent> fused strain, return mapping, tangent and forces",
     "constitutive_S": "k_mc3d return mapping (stress only)",
     "assembly": "tangent assembly (B'DB into the block pattern)",
     "amg_update": "AMG numeric value update (sequence of kernels per Newton iteration)",
     "amg_vcycle": "AMG V-cycle (sequence of kernels per application)",
     "spmv3_f16": "k_spmv_h3 FP16 level-0 copy",
     "spmv3_f64_aorth": "k_spmv_blk 3x3 FP64 inside the A-orthogonalisation",
-    "residual": "k_residual3d fused stress-only residual",
+    "residual": "k_response3d fused stress-only residual",
     "spmm3_f64_aorth": "k_spmm3 FP64 multi-vector SpMM of the A-orthogonalisation",
-    "a_orthogonalize": "whole A-orthogonalisation of the deflation basis (SpMM + blocked Gram-Schmidt)",
+    "a_orthogonalize": "whole A-orthogonalisation of the deflation basis (SpMM, Gram matrix, products)",
 }
 
 
 def kind_bytes(P, amg, units=None, launches=None):
     """Algorithmic bytes per launch of every instrumented kind (each operand read once, each
     result written once).  SpMV: values + block columns + row pointers + x read + y written;
-    return map 416 B (S and DS) or 128 B (S) per point; assembly 5,896 B per element + the K
-    values written; fused residual 280 B per point + U gathered and F written once; AMG
+    fused residual per point nine gradient factors, four fields and the weight (112 B), with the
+    tangent 384 B more (E, S, DS written), U gathered and F written once; return map alone 128 B (S)
+    per point; assembly DS, factors and weights of the eleven points (4,048 B) per element + the K
+    values written; AMG
     update: the fine matrix read (and its FP32 copy written in the mixed form), every level's
     P and R written, every coarse matrix written; V-cycle: per level six smoother/residual
     SpMVs and the two transfers, the coarsest dense solve."""
@@ -764,8 +766,8 @@ def kind_bytes(P, amg, units=None, launches=None):
     return {"spmv3_f64": spmv64, "spmv3_f64_aorth": spmv64, "spmm3_f64_aorth": spmm,
             "spmv3_f32": nb * (36 + 4) + (nr + 1) * 4 + 3 * 4 * nd,
             "spmv3_f16": nb * (24 + 4) + (nr + 1) * 4 + 3 * 4 * nd,
-            "constitutive_S_DS": ni * 416, "constitutive_S": ni * 128,
-            "assembly": ne * 5896 + nb * 72, "residual": ni * 280 + ne * 30 * 8 + nd * 8,
+            "constitutive_S_DS": ni * 496 + ne * 30 * 8 + nd * 8, "constitutive_S": ni * 128,
+            "assembly": ne * 4048 + nb * 72, "residual": ni * 112 + ne * 30 * 8 + nd * 8,
             "amg_update": upd, "amg_vcycle": cyc, "a_orthogonalize": None}
 
 

@@ -7,7 +7,8 @@
 //       two passes of one multi-dot and one GEMV each) instead of the reference's modified
 //       Gram-Schmidt loop -- the same projection with MGS-level stability in 4 sweeps
 //       over the basis instead of 2(j+1).  The small least-squares problem is solved with
-//       Givens rotations on the host (the reference re-solves H \ g each step; same y).
+//       Givens rotations, on the device in the replayed loop and on the host in the other (the
+//       reference re-solves H \ g each step; same y).
 //   sg_a_orthogonalize   +LINEAR_SOLVERS/A_orthogonalize.m:1-58 (columns processed last
 //       to first, one-pass A-orthogonalisation against the kept columns, columns with
 //       |w'Aw| <= eps dropped, output reversed)
@@ -669,7 +670,7 @@ extern "C" int sg_a_orthogonalize(sg_krylov *ws, const sg_bsr *A, const double *
     }
     if (rc) return rc;
     if (ws->aorth_mode == 1) {
-        // Gram matrix, recurrence on one CTA, then U = S T into Wo and A U = (A S) T into AW
+        // Gram matrix, recurrence on one CTA, then U = S T and A U = (A S) T (in place, or through Wo into W and AW)
         if (!ws->gpart) {
             SG_CUDA(device_alloc(&ws->gpart, sizeof(double) * GR_CTAS * 64 * 64));
             SG_CUDA(device_alloc(&ws->gkout, sizeof(int32_t) * 4));

@@ -18,8 +18,8 @@ The A-orthogonalisation runs against the assembled tangent of the seeded points,
 kernels on the elastic stiffness of the draws' moduli.
 
 Per kernel it prints one JSON line: mean time per launch and the algorithmic bytes per
-launch (return mapping: 416 B per point with the tangent, 128 B without; assembly: 5,896 B
-per element + 8 B per stored value; SpMV: 76 B per 3x3 block + row pointers + x and y), the
+launch (return mapping: 416 B per point with the tangent, 128 B without; assembly: 4,048 B
+per P2 tetrahedron + 8 B per stored value; SpMV: 76 B per 3x3 block + row pointers + x and y), the
 achieved GB/s and its fraction of the measured copy bandwidth.  Every operand is larger than
 the 126 MB L2, so launches need no flush in between.
 """
@@ -125,8 +125,8 @@ def main(argv=None):
     specs = {
         "sds": (sds, n * 416, "k_mc3d (S and DS)"),
         "s": (s_only, n * 128, "k_mc3d (S only)"),
-        "assembly": (lambda: dm.assemble(DS, K), dm.n_e * 5896 + nnz_vals * 8,
-                     "k_element_blocks_p2tet + k_gather_blocks3" if dm.tangent_fused else "k_assemble_bsr"),
+        "assembly": (lambda: dm.assemble(DS, K), dm.n_e * 4048 + nnz_vals * 8,
+                     "k_element_blocks_fact + k_gather_upper" if dm.tangent_fused else "k_assemble_bsr"),
         "spmv": (lambda: dm.spmv(K, x, y), dm.n_blocks * 76 + (dm.n_n + 1) * 4 + 16 * dm.n_dof,
                  "k_spmv_blk 3x3"),
     }
