@@ -58,8 +58,8 @@ struct sg_krylov {
     bool gproj = false;         // the captured loop forms A z for the projection
     int64_t launches_start = 0, launches_body = 0, launches_end = 0;
     int use_graph = 1;
-    // blocked A-orthogonalisation: A times the block's input columns (n x 16), the block's
-    // coefficients against earlier columns (256 x 16) and the per-CTA partial sums
+    // blocked A-orthogonalisation (aorth_mode 0, allocated on its first use): A times the block's input
+    // columns (n x 16), the block's coefficients against earlier columns (256 x 16) and the per-CTA partial sums
     double *atb = nullptr, *cblk = nullptr, *tspart = nullptr;
     // Gram-matrix A-orthogonalisation (default, aorth_mode 1): G, T, the output-ordered T and
     // the output columns' processing indices (3 kcap^2 + kcap), the Gram partial sums
@@ -457,10 +457,13 @@ extern "C" int sg_krylov_create(int64_t n, int32_t maxit, sg_krylov **out) {
     if (!e) e = sg::device_alloc(&ws->w, sizeof(double) * n);
     if (!e) e = sg::device_alloc(&ws->t, sizeof(double) * n);
     if (!e) e = sg::device_alloc(&ws->hdev, sizeof(double) * (2 * (maxit + 2) + 8));
+    if (!e) e = sg::device_alloc(&ws->gpart, sizeof(double) * GR_CTAS * 64 * 64);
+    if (!e) e = sg::device_alloc(&ws->gkout, sizeof(int32_t) * 4);
     if (!e) e = cudaMallocHost(&ws->hpin, sizeof(double) * (2 * (maxit + 2) + 8));
     int rc = e ? cuda_error(e, "Krylov workspace") : ensure_kcap(ws, 16);
     if (rc) {
         cudaFree(ws->V); cudaFree(ws->Z); cudaFree(ws->w); cudaFree(ws->t); cudaFree(ws->hdev);
+        cudaFree(ws->gpart); cudaFree(ws->gkout);
         if (ws->hpin) cudaFreeHost(ws->hpin);
         delete ws;
         return rc;
@@ -655,13 +658,8 @@ extern "C" int sg_a_orthogonalize(sg_krylov *ws, const sg_bsr *A, const double *
     // products do not depend on the orthogonalisation, and one SpMM reads A once per eight
     // columns where a SpMV per column reads it k times
     if (A->b == 3 && k >= 4) {
-        // interleaved copies of 16 columns (scratch: the block buffer)
-        if (!ws->atb) {
-            SG_CUDA(device_alloc(&ws->atb, sizeof(double) * n * 16));
-            SG_CUDA(device_alloc(&ws->cblk, sizeof(double) * 256 * 16));
-            SG_CUDA(device_alloc(&ws->tspart, sizeof(double) * TS_PART_CTAS * 256 * 16));
-        }
-        rc = bsr_spmm_interleaved(*A, Avals, W + (int64_t)(k - 1) * n, -n, AWo, n, k, ws->atb, st);
+        // interleaved copies of 16 columns in Wo, which holds nothing yet (kcap >= 64 columns)
+        rc = bsr_spmm_interleaved(*A, Avals, W + (int64_t)(k - 1) * n, -n, AWo, n, k, Wo, st);
     } else if (A->b == 3) {
         rc = bsr_spmm(*A, Avals, W + (int64_t)(k - 1) * n, -n, AWo, n, k, st);
     } else {
@@ -671,10 +669,6 @@ extern "C" int sg_a_orthogonalize(sg_krylov *ws, const sg_bsr *A, const double *
     if (rc) return rc;
     if (ws->aorth_mode == 1) {
         // Gram matrix, recurrence on one CTA, then U = S T and A U = (A S) T (in place, or through Wo into W and AW)
-        if (!ws->gpart) {
-            SG_CUDA(device_alloc(&ws->gpart, sizeof(double) * GR_CTAS * 64 * 64));
-            SG_CUDA(device_alloc(&ws->gkout, sizeof(int32_t) * 4));
-        }
         double *G = ws->gram, *Tp = G + (int64_t)k * k, *Ta = Tp + (int64_t)k * k;
         int32_t *pmap = reinterpret_cast<int32_t *>(Ta + (int64_t)k * k);
         const double *S = W + (int64_t)(k - 1) * n;   // processing order: column i is W's k - 1 - i
