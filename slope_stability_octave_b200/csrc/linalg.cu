@@ -495,7 +495,19 @@ __device__ __forceinline__ void spmm_columns_out(const double *sY, int nr, int64
     }
 }
 
-template <int KC>
+// s += v, and e += the rounding error of that sum.  Exact where |s| >= |v|; where a block outweighs the
+// sum so far, off by at most a rounding of the block itself.  Four operations (Knuth's two-sum takes
+// seven: 1.24 against 1.22 ms for 21 columns of 6.1M blocks, its errors 2 % lower).
+__device__ __forceinline__ void add_kept(double &s, double &e, double v) {
+    const double n = s + v;
+    e += v - (n - s);
+    s = n;
+}
+// the error to add at the end; none (the plain sum then) where the sum met an infinity
+__device__ __forceinline__ double kept_error(double e) { return isfinite(e) ? e : 0.0; }
+
+// KEEP: a lane's sum over the row's blocks carries its rounding error along (bsr_spmm_interleaved).
+template <int KC, bool KEEP>
 __global__ void __launch_bounds__(256) k_spmm3i(int64_t nrows, int64_t rows_per_cta, const int32_t *__restrict__ rp,
                                                 const int32_t *__restrict__ col, const double *__restrict__ vals,
                                                 const double *__restrict__ Xi, int kc, double *__restrict__ Y,
@@ -512,6 +524,7 @@ __global__ void __launch_bounds__(256) k_spmm3i(int64_t nrows, int64_t rows_per_
     const int64_t rend = r0 + rows_per_cta < nrows ? r0 + rows_per_cta : nrows;
     for (int64_t row = r0 + (threadIdx.x >> 5); row < rend; row += blockDim.x >> 5) {
         double y0 = 0.0, y1 = 0.0, y2 = 0.0;
+        double e0 = 0.0, e1 = 0.0, e2 = 0.0;
         const int32_t p1 = rp[row + 1];
         for (int32_t p0 = rp[row]; p0 < p1; p0 += NS) {
             const int32_t p = p0 + bs;
@@ -534,9 +547,23 @@ __global__ void __launch_bounds__(256) k_spmm3i(int64_t nrows, int64_t rows_per_
 #pragma unroll
             for (int t = 0; t < 8; ++t) a[t] = __shfl_sync(0xffffffffu, av, base + t);
             a[8] = KC == 8 ? __shfl_sync(0xffffffffu, a8, base) : __shfl_sync(0xffffffffu, av, base + 8);
-            y0 += a[0] * u0 + a[1] * u1 + a[2] * u2;
-            y1 += a[3] * u0 + a[4] * u1 + a[5] * u2;
-            y2 += a[6] * u0 + a[7] * u1 + a[8] * u2;
+            const double b0 = a[0] * u0 + a[1] * u1 + a[2] * u2;
+            const double b1 = a[3] * u0 + a[4] * u1 + a[5] * u2;
+            const double b2 = a[6] * u0 + a[7] * u1 + a[8] * u2;
+            if constexpr (KEEP) {
+                add_kept(y0, e0, b0);
+                add_kept(y1, e1, b1);
+                add_kept(y2, e2, b2);
+            } else {
+                y0 += b0;
+                y1 += b1;
+                y2 += b2;
+            }
+        }
+        if constexpr (KEEP) {
+            y0 += kept_error(e0);
+            y1 += kept_error(e1);
+            y2 += kept_error(e2);
         }
 #pragma unroll
         for (int off = KC; off < 32; off <<= 1) {
@@ -570,7 +597,11 @@ __global__ void __launch_bounds__(256) k_spmm3i(int64_t nrows, int64_t rows_per_
 // block row as three of eight tile rows, values straight into the fragments (2.0-2.4 ms: fewer
 // instructions, but twice the requests for the values), rows in bricks of 2 to 8 nodes a side
 // (1.67-2.0 ms: the gathers already hit L2, and its rate is not the bound).
-__global__ void __launch_bounds__(256, 4) k_spmm3p(int64_t nrows, int64_t rows_per_cta,
+// KEEP: the two groups' products of a step are added first and join a sum that carries its
+// rounding error along (bsr_spmm_interleaved says where).  Twelve more values a lane: three
+// CTAs of 80 registers (four of 64 spill them: 1.47 against 1.22 ms for 21 columns of 6.1M blocks).
+template <bool KEEP>
+__global__ void __launch_bounds__(256, KEEP ? 3 : 4) k_spmm3p(int64_t nrows, int64_t rows_per_cta,
                                                 const int32_t *__restrict__ rp, const int32_t *__restrict__ col,
                                                 const double *__restrict__ vals, const double *__restrict__ Xi, int kc,
                                                 double *__restrict__ Y, int64_t ldy) {
@@ -581,6 +612,7 @@ __global__ void __launch_bounds__(256, 4) k_spmm3p(int64_t nrows, int64_t rows_p
     const int64_t rend = r0 + rows_per_cta < nrows ? r0 + rows_per_cta : nrows;
     for (int64_t row = r0 + (threadIdx.x >> 5); row < rend; row += blockDim.x >> 5) {
         double y[3][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+        double err[3][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
         const int32_t p1 = rp[row + 1];
         for (int32_t p0 = rp[row]; p0 < p1; p0 += NS * UNR) {
             int64_t j[UNR];
@@ -600,6 +632,7 @@ __global__ void __launch_bounds__(256, 4) k_spmm3p(int64_t nrows, int64_t rows_p
                 }
             }
             double2 u[UNR][3];
+            double step[3][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
 #pragma unroll
             for (int q = 0; q < UNR; ++q) {
                 u[q][0] = u[q][1] = u[q][2] = make_double2(0.0, 0.0);
@@ -618,9 +651,24 @@ __global__ void __launch_bounds__(256, 4) k_spmm3p(int64_t nrows, int64_t rows_p
                 a[8] = __shfl_sync(0xffffffffu, a8[q], base);
 #pragma unroll
                 for (int r = 0; r < 3; ++r) {
-                    y[r][0] += a[3 * r] * u[q][0].x + a[3 * r + 1] * u[q][1].x + a[3 * r + 2] * u[q][2].x;
-                    y[r][1] += a[3 * r] * u[q][0].y + a[3 * r + 1] * u[q][1].y + a[3 * r + 2] * u[q][2].y;
+                    double(&to)[2] = KEEP ? step[r] : y[r];
+                    to[0] += a[3 * r] * u[q][0].x + a[3 * r + 1] * u[q][1].x + a[3 * r + 2] * u[q][2].x;
+                    to[1] += a[3 * r] * u[q][0].y + a[3 * r + 1] * u[q][1].y + a[3 * r + 2] * u[q][2].y;
                 }
+            }
+            if constexpr (KEEP) {
+#pragma unroll
+                for (int r = 0; r < 3; ++r) {
+                    add_kept(y[r][0], err[r][0], step[r][0]);
+                    add_kept(y[r][1], err[r][1], step[r][1]);
+                }
+            }
+        }
+        if constexpr (KEEP) {
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                y[r][0] += kept_error(err[r][0]);
+                y[r][1] += kept_error(err[r][1]);
             }
         }
 #pragma unroll
@@ -642,11 +690,19 @@ __global__ void __launch_bounds__(256, 4) k_spmm3p(int64_t nrows, int64_t rows_p
     spmm_columns_out(&sY[0][0], (int)(rend - r0) * 3, r0 * 3, kc, Y, ldy);
 }
 
-int bsr_spmm_interleaved(const sg_bsr &A, const double *vals, const double *X, int64_t ldx, double *Y, int64_t ldy,
-                         int k, double *Xi, cudaStream_t st) {
-    if (A.b != 3) return set_error(SG_ERR_ARG, "bsr_spmm: 3x3 blocks only");
+// Up to this many unknowns the sums carry their rounding errors.  Their rows were summed by a lane
+// per block and a shuffle tree before they came here (from 4 columns on); four lanes with seven
+// blocks each in series would round more.  Relative error of A S T against long double, 21 columns:
+// 0.63M unknowns 1.77e-15 with the tree, 1.89e-15 in series, 1.67e-15 as it is; 82k unknowns 5.2e-16,
+// 5.6e-16, 5.0e-16.  It takes 0.16 of the 1.22 ms of such a call.  Larger meshes have had the serial
+// sums all along (there it would add 1.1 to 6.7 ms).
+constexpr int64_t SPMM_KEEP_MAX = 750000;
+
+template <bool KEEP>
+static int spmm_interleaved(const sg_bsr &A, const double *vals, const double *X, int64_t ldx, double *Y, int64_t ldy,
+                            int k, double *Xi, cudaStream_t st) {
     const int64_t n = A.n_rows * 3;
-    // 16 columns per pass; a last pass of at most 8 columns takes half the gathered bytes and MMAs
+    // 16 columns per pass; a last pass of at most 8 columns takes half the gathered bytes
     for (int c0 = 0; c0 < k;) {
         const int rest = k - c0;
         const int KC = rest > 8 ? 16 : 8;
@@ -659,16 +715,23 @@ int bsr_spmm_interleaved(const sg_bsr &A, const double *vals, const double *X, i
         const unsigned gr = grid_chunks(A.n_rows, rpc);
         if (KC == 16) {
             k_pack_tiles<16><<<gt, 256, 0, st>>>(n, kc, X + c0 * ldx, ldx, Xi);
-            k_spmm3p<<<gr, 256, 0, st>>>(A.n_rows, rpc, A.d_row_ptr, A.d_col, vals, Xi, kc, Y + c0 * ldy, ldy);
+            k_spmm3p<KEEP><<<gr, 256, 0, st>>>(A.n_rows, rpc, A.d_row_ptr, A.d_col, vals, Xi, kc, Y + c0 * ldy, ldy);
         } else {
             k_pack_tiles<8><<<gt, 256, 0, st>>>(n, kc, X + c0 * ldx, ldx, Xi);
-            k_spmm3i<8><<<gr, 256, 0, st>>>(A.n_rows, rpc, A.d_row_ptr, A.d_col, vals, Xi, kc, Y + c0 * ldy, ldy);
+            k_spmm3i<8, KEEP><<<gr, 256, 0, st>>>(A.n_rows, rpc, A.d_row_ptr, A.d_col, vals, Xi, kc, Y + c0 * ldy, ldy);
         }
         instr_end(tk, st);
         SG_CUDA(cudaGetLastError());
         c0 += kc;
     }
     return SG_OK;
+}
+
+int bsr_spmm_interleaved(const sg_bsr &A, const double *vals, const double *X, int64_t ldx, double *Y, int64_t ldy,
+                         int k, double *Xi, cudaStream_t st) {
+    if (A.b != 3) return set_error(SG_ERR_ARG, "bsr_spmm: 3x3 blocks only");
+    return A.n_rows * 3 <= SPMM_KEEP_MAX ? spmm_interleaved<true>(A, vals, X, ldx, Y, ldy, k, Xi, st)
+                                         : spmm_interleaved<false>(A, vals, X, ldx, Y, ldy, k, Xi, st);
 }
 
 int bsr_spmm(const sg_bsr &A, const double *vals, const double *X, int64_t ldx, double *Y, int64_t ldy, int k,
