@@ -499,12 +499,7 @@ static int element_blocks(sg_mesh *m, const double *DS, cudaStream_t st) {
                            reinterpret_cast<uintptr_t>(m->d_w)) & 15) == 0;
     int32_t *status = device_status_word();
     if (aligned && status && smem_bulk <= 113 * 1024) {
-        static thread_local size_t configured_bulk = 0;
-        if (smem_bulk > configured_bulk) {
-            SG_CUDA(cudaFuncSetAttribute(k_element_blocks_p2tet_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem_bulk));
-            configured_bulk = smem_bulk;
-        }
+        SG_CUDA(allow_dynamic_smem(k_element_blocks_p2tet_bulk, smem_bulk));
         count_launch();
         const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(batches, (int64_t)sm_count() * 2));
         k_element_blocks_p2tet_bulk<<<grid, KE_EPB * KE_TPE, smem_bulk, st>>>(m->n_e, m->nq, m->d_dphi, m->d_w, DS,
@@ -513,11 +508,7 @@ static int element_blocks(sg_mesh *m, const double *DS, cudaStream_t st) {
         return SG_OK;
     }
     const size_t smem = sizeof(double) * (size_t)KE_EPB * m->nq * (36 + 30 + 1);
-    static thread_local size_t configured = 0;
-    if (smem > configured) {
-        SG_CUDA(cudaFuncSetAttribute(k_element_blocks_p2tet, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured = smem;
-    }
+    SG_CUDA(allow_dynamic_smem(k_element_blocks_p2tet, smem));
     count_launch();
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(batches, (int64_t)sm_count() * 8));
     k_element_blocks_p2tet<<<grid, KE_EPB * KE_TPE, smem, st>>>(m->n_e, m->nq, m->d_dphi, m->d_w, DS, m->d_ke);

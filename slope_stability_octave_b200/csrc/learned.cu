@@ -752,14 +752,7 @@ __global__ void k_features(int64_t nn, int64_t n_pad, const int32_t *__restrict_
 int mlp_launch(int mode, const float *params, const uint16_t *X, int64_t n, float *G, const float *dG, float *part,
                int nparts, int *err, cudaStream_t st) {
     const int64_t ntiles = (n + TILE - 1) / TILE;
-    static int attr_done[2] = {0, 0};
-    if (!attr_done[mode]) {
-        if (mode == 0)
-            SG_CUDA(cudaFuncSetAttribute(k_mlp<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
-        else
-            SG_CUDA(cudaFuncSetAttribute(k_mlp<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
-        attr_done[mode] = 1;
-    }
+    SG_CUDA(mode == 0 ? allow_dynamic_smem(k_mlp<0>, SMEM_BYTES) : allow_dynamic_smem(k_mlp<1>, SMEM_BYTES));
     count_launch();
     if (mode == 0)
         k_mlp<0><<<nparts, 128, SMEM_BYTES, st>>>(params, X, n, ntiles, G, nullptr, nullptr, err);

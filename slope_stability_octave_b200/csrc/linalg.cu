@@ -1229,11 +1229,7 @@ static int gram_direct(int64_t n, int k, const double *S, int64_t lds, const dou
                        cudaStream_t st) {
     constexpr int stages = GD_STAGES * 2 * 8 * NB * GD_LD, sums = GD_WARPS * NB * (NB + 1) / 2 * 64;
     constexpr size_t smem = sizeof(double) * (stages > sums ? stages : sums);
-    static thread_local bool configured = false;
-    if (!configured) {
-        SG_CUDA(cudaFuncSetAttribute(k_gram_direct<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured = true;
-    }
+    SG_CUDA(allow_dynamic_smem(k_gram_direct<NB>, smem));
     k_gram_direct<NB><<<GR_CTAS, GD_THREADS, smem, st>>>(n, k, S, lds, AS, ldas, part);
     SG_CUDA(cudaGetLastError());
     return SG_OK;
@@ -1360,12 +1356,7 @@ int gram_upper(int64_t n, int k, const double *S, int64_t lds, const double *AS,
         SG_CUDA(cudaGetLastError());
         return SG_OK;
     }
-    static thread_local bool configured = false;
-    if (!configured) {   // the stages exceed the default 48 KB
-        SG_CUDA(cudaFuncSetAttribute(k_gram_partial_mma, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)GM_SMEM));
-        configured = true;
-    }
+    SG_CUDA(allow_dynamic_smem(k_gram_partial_mma, GM_SMEM));
     const int TW = GM_TW, nt = (k + TW - 1) / TW;
     for (int p = 0; p < nt; ++p)
         for (int q = 0; q <= p; ++q) {
@@ -1384,11 +1375,7 @@ int gram_recurrence(int k, const double *G, double *Tp, double eps, double *Ta, 
     const size_t full = base + sizeof(double) * 2 * (size_t)k * k;
     const bool staged = full <= 200 * 1024;
     const size_t smem = staged ? full : base;
-    static thread_local size_t configured = 0;
-    if (smem > 48 * 1024 && smem > configured) {
-        SG_CUDA(cudaFuncSetAttribute(k_gram_recurrence, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured = smem;
-    }
+    SG_CUDA(allow_dynamic_smem(k_gram_recurrence, smem));
     count_launch();
     k_gram_recurrence<<<1, 256, smem, st>>>(k, G, Tp, eps, Ta, nt, sig, kout, pmap, staged ? 1 : 0);
     SG_CUDA(cudaGetLastError());
@@ -1577,9 +1564,9 @@ int ts_apply(int64_t n, int k, const int32_t *kout, const int32_t *pmap, const d
              const double *Ta, double *Y, int64_t ldy, cudaStream_t st) {
     if (k <= 0 || n <= 0) return SG_OK;
     const int64_t ntiles = (n + TA_R - 1) / TA_R;
+    SG_CUDA(allow_dynamic_smem(k_ts_apply_mma, TM_SMEM));
     static thread_local int resident_mma = 0;
     if (!resident_mma) {
-        SG_CUDA(cudaFuncSetAttribute(k_ts_apply_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TM_SMEM));
         int r = 0;
         SG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_ts_apply_mma, 256, TM_SMEM));
         resident_mma = std::max(1, r);

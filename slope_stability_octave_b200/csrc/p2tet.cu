@@ -220,6 +220,7 @@ constexpr int RSP_TP = 13;                       // doubles per point of the tra
 constexpr int RSP_DSP = 37, RSP_SP = 7;          // staging pitches of DS and of E, S
 constexpr size_t RSP_SMEM = sizeof(double) * (RSP_EL * 30 + RSP_THREADS * RSP_TP + RSP_EL * 48);
 constexpr size_t RSP_SMEM_DS = RSP_SMEM + sizeof(double) * RSP_WARPS * 32 * (RSP_DSP + RSP_SP);
+static_assert(RSP_SMEM_DS <= 48 * 1024, "within the default limit of dynamic shared memory");
 
 // NQ > 0: the rule's size at compile time (its table then sits in the instructions' constant operands).
 template <bool TANGENT, bool FACT, int NQ>
@@ -512,14 +513,6 @@ static int launch_response(const sg_mesh *m, ResponseArgs A, int kind, cudaStrea
         const bool fact = m->d_gxi != nullptr, r11 = fact && m->nq == P2T_REF_RULE;
         const size_t smem = tangent ? RSP_SMEM_DS : RSP_SMEM;
         if (tangent) {
-            static thread_local bool configured = false;
-            if (!configured) {   // the stage of DS exceeds the default 48 KB
-                const auto opt = cudaFuncAttributeMaxDynamicSharedMemorySize;
-                SG_CUDA(cudaFuncSetAttribute(k_response3d<true, true, P2T_REF_RULE>, opt, (int)RSP_SMEM_DS));
-                SG_CUDA(cudaFuncSetAttribute(k_response3d<true, true, 0>, opt, (int)RSP_SMEM_DS));
-                SG_CUDA(cudaFuncSetAttribute(k_response3d<true, false, 0>, opt, (int)RSP_SMEM_DS));
-                configured = true;
-            }
             if (r11) k_response3d<true, true, P2T_REF_RULE><<<grid, RSP_THREADS, smem, st>>>(A, rule);
             else if (fact) k_response3d<true, true, 0><<<grid, RSP_THREADS, smem, st>>>(A, rule);
             else k_response3d<true, false, 0><<<grid, RSP_THREADS, smem, st>>>(A, rule);
@@ -786,20 +779,13 @@ int p2tet_element_blocks(const sg_mesh *m, const double *DS, double *Ke, cudaStr
     P2TetMoments mom;
     for (int q = 0; q < EB_NQ; ++q)
         for (int i = 0; i < 10; ++i) mom.c[q][i] = m->rule[q][eb_s(i)] * m->rule[q][eb_t(i)];
-    static thread_local bool configured = false;
-    if (!configured) {
-        const auto opt = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        SG_CUDA(cudaFuncSetAttribute(k_element_blocks_fact<true>, opt, (int)EB_SMEM));
-        SG_CUDA(cudaFuncSetAttribute(k_element_blocks_fact<false>, opt, (int)EB_SMEM));
-        configured = true;
-    }
     const int64_t passes = (m->n_e + EB_EL - 1) / EB_EL;
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(passes, (int64_t)sm_count() * 3));
     count_launch();
-    if ((reinterpret_cast<uintptr_t>(DS) & 15) == 0)
-        k_element_blocks_fact<true><<<grid, EB_THREADS, EB_SMEM, st>>>(m->n_e, m->d_gxi, m->d_w, DS, mom, Ke);
-    else
-        k_element_blocks_fact<false><<<grid, EB_THREADS, EB_SMEM, st>>>(m->n_e, m->d_gxi, m->d_w, DS, mom, Ke);
+    const auto kernel = (reinterpret_cast<uintptr_t>(DS) & 15) == 0 ? k_element_blocks_fact<true>
+                                                                     : k_element_blocks_fact<false>;
+    SG_CUDA(allow_dynamic_smem(kernel, EB_SMEM));
+    kernel<<<grid, EB_THREADS, EB_SMEM, st>>>(m->n_e, m->d_gxi, m->d_w, DS, mom, Ke);
     SG_CUDA(cudaGetLastError());
     return SG_OK;
 }

@@ -7,6 +7,7 @@
 #include <string>
 
 #include "../../include/slopegpu.h"
+#include "dyn_smem.h"
 
 namespace sg {
 
