@@ -551,8 +551,10 @@ __device__ __forceinline__ void davis_reduce(double c0, double phi, double psi, 
                                              double &c_bar, double &sin_phi) {
     // u = tan of the reduced friction angle.  The reference takes cos and sin of arctangents;
     // with t = tan(f), f in (-pi/2, pi/2): cos f = 1 / sqrt(1 + t^2), sin f = t cos f.
+    // The squares of tangents must not overflow; from lambda = 1e-140 down the results for phi > 0 have
+    // long reached their limits.
     double beta, c_l, u;
-    const double inv = 1.0 / lambda;
+    const double inv = fmin(1.0 / lambda, 1e140);
     if (type == 'A') {
         double sf, cf, ss = 0.0, cs = 1.0;
         sincos(phi, &sf, &cf);
