@@ -133,6 +133,10 @@ int sg_mesh_create(int dim, int32_t n_p, int32_t n_q, int64_t n_n, int64_t n_e, 
 int sg_mesh_destroy(sg_mesh *mesh);
 /* sizes[0..4] = n_dof (dim*n_n), n_Q, nnz of K(Q,Q), BSR blocks, n_int */
 int sg_mesh_sizes(const sg_mesh *mesh, int64_t *sizes);
+/* *factored = 1 when the mesh's gradients were found to be those of isoparametric P2
+ * tetrahedra in the reference's local numbering, so that the element kernels work on the
+ * three barycentric gradients of a point; 0: they read the ten basis gradients. */
+int sg_mesh_factored(const sg_mesh *mesh, int32_t *factored);
 /* borrowed pointer to the mesh's block pattern (valid until sg_mesh_destroy) */
 int sg_mesh_bsr(const sg_mesh *mesh, const sg_bsr **bsr);
 /* (b1) ref_I, ref_J: 1-based pattern of K(Q,Q) in find() order; transpose_perm: 1-based

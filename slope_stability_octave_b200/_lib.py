@@ -34,6 +34,7 @@ SIGNATURES = {
     # mesh and element operators
     "sg_mesh_create": [cint, i32, i32, i64, i64, vp, vp, vp, vp, vp, vp, vp],
     "sg_mesh_destroy": [vp],
+    "sg_mesh_factored": [vp, vp],
     "sg_mesh_sizes": [vp, vp],
     "sg_mesh_bsr": [vp, vp],
     "sg_mesh_pattern": [vp, vp, vp, vp],

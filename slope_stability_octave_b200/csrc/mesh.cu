@@ -332,6 +332,12 @@ extern "C" int sg_mesh_sizes(const sg_mesh *m, int64_t *sizes) {
     return SG_OK;
 }
 
+extern "C" int sg_mesh_factored(const sg_mesh *m, int32_t *factored) {
+    SG_CHECK_ARG(m && factored, "null argument");
+    *factored = m->d_gxi != nullptr;
+    return SG_OK;
+}
+
 extern "C" int sg_mesh_bsr(const sg_mesh *m, const sg_bsr **bsr) {
     SG_CHECK_ARG(m && bsr, "null argument");
     *bsr = &m->bsr;

@@ -130,6 +130,13 @@ class DeviceMesh:
         _lib.call("sg_force_dev", self.handle, ptr(S), int(s_rows), ptr(F), cur_stream())
 
     @property
+    def factored(self):
+        """Whether the element kernels work on the factored gradients of P2 tetrahedra."""
+        out = C.c_int32()
+        _lib.call("sg_mesh_factored", self.handle, C.byref(out))
+        return bool(out.value)
+
+    @property
     def fused_residual(self):
         """The fused stress-only residual kernel covers P2 tetrahedra."""
         return self.dim == 3 and self.mesh.elem.shape[0] == 10
