@@ -655,8 +655,8 @@ extern "C" int sg_a_orthogonalize(sg_krylov *ws, const sg_bsr *A, const double *
     double *nt = ws->nt, *sig = ws->sig;
     const unsigned gb = grid_for(n, 256, 8);
     // A times every input column up front (processing order i takes column k - 1 - i): the
-    // products do not depend on the orthogonalisation, and one SpMM reads A once per eight
-    // columns where a SpMV per column reads it k times
+    // products do not depend on the orthogonalisation, and a product with several columns reads A
+    // once for all of them (16 from four columns on)
     if (A->b == 3 && k >= 4) {
         // interleaved copies of 16 columns in Wo, which holds nothing yet (kcap >= 64 columns)
         rc = bsr_spmm_interleaved(*A, Avals, W + (int64_t)(k - 1) * n, -n, AWo, n, k, Wo, st);

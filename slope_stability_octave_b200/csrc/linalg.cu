@@ -740,20 +740,17 @@ int bsr_spmm(const sg_bsr &A, const double *vals, const double *X, int64_t ldx, 
     const double avg = A.n_rows > 0 ? (double)A.n_blocks / (double)A.n_rows : 8.0;
     // the same lanes per row as the single-vector SpMV (bitwise-equal columns)
     const int G = avg >= 16.0 ? 32 : (avg >= 8.0 ? 16 : 8);
-    // Columns per pass: every block row gathers x entries of its ~28 neighbours from each
-    // column, so the pass's input vectors must stay resident in L2 (126 MB) to be read from
-    // DRAM about once; keep them within ~48 MB (8 columns on meshes up to 0.6M nodes, 2 on the
-    // 3M-DOF slope) and read the matrix once per pass.
+    // Columns per pass (a basis of one to three columns comes here): the x entries that the rows
+    // gather stay in L2 while a pass's input vectors take no more than 48 MB of it.
     const double vec_bytes = 8.0 * (double)A.n_rows * 3;
-    const int kcmax = vec_bytes * 8 <= 48e6 ? 8 : (vec_bytes * 4 <= 48e6 ? 4 : (vec_bytes * 2 <= 48e6 ? 2 : 1));
+    const int kcmax = vec_bytes * 4 <= 48e6 ? 4 : (vec_bytes * 2 <= 48e6 ? 2 : 1);
     for (int c0 = 0; c0 < k; c0 += kcmax) {
         const int kc = std::min(kcmax, k - c0);
         const InstrToken tk = instr_begin(IK_SPMM_AORTH, st);
         instr_units(IK_SPMM_AORTH, kc);
         const double *Xc = X + c0 * ldx;
         double *Yc = Y + c0 * ldy;
-        if (kcmax == 8) spmm_pass<8>(A, G, vals, Xc, ldx, Yc, ldy, kc, st);
-        else if (kcmax == 4) spmm_pass<4>(A, G, vals, Xc, ldx, Yc, ldy, kc, st);
+        if (kcmax == 4) spmm_pass<4>(A, G, vals, Xc, ldx, Yc, ldy, kc, st);
         else spmm_pass<2>(A, G, vals, Xc, ldx, Yc, ldy, kc, st);
         instr_end(tk, st);
         SG_CUDA(cudaGetLastError());

@@ -38,7 +38,7 @@ int cheb_step(int b, int64_t nrows, int64_t nblk, const int32_t *rp, const int32
               const T *rhs, const ChebStep<T> &step, cudaStream_t st);
 
 // Y(:, c) = A X(:, c) for c < k, FP64 3x3 blocks; X, Y column-major (leading dimensions may
-// be negative).  Reads the matrix once per 8 columns; each column equals bsr_spmv's bitwise.
+// be negative).  For up to three columns; each column equals bsr_spmv's bitwise.
 int bsr_spmm(const sg_bsr &A, const double *vals, const double *X, int64_t ldx, double *Y, int64_t ldy, int k,
              cudaStream_t st);
 
