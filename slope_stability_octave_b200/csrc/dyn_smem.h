@@ -4,12 +4,11 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
-#include <vector>
-
 namespace sg {
 
 // Raises the kernel's limit on the current device to `bytes`.  The limit belongs to the device, so
-// what has been raised is remembered by (kernel, device); each host thread keeps its own list.
+// what has been raised is remembered by (kernel, device); each host thread keeps its own list (a full
+// list asks the driver each time).
 inline cudaError_t allow_dynamic_smem(const void *kernel, size_t bytes) {
     if (bytes <= 48 * 1024) return cudaSuccess;
     struct Raised {
@@ -17,18 +16,19 @@ inline cudaError_t allow_dynamic_smem(const void *kernel, size_t bytes) {
         int device;
         size_t bytes;
     };
-    static thread_local std::vector<Raised> raised;
+    constexpr int most = 64;
+    static thread_local Raised raised[most];
+    static thread_local int count = 0;
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
-    Raised *at = nullptr;
-    for (Raised &r : raised)
-        if (r.kernel == kernel && r.device == device) at = &r;
-    if (at && bytes <= at->bytes) return cudaSuccess;
+    int at = 0;
+    while (at < count && !(raised[at].kernel == kernel && raised[at].device == device)) ++at;
+    if (at < count && bytes <= raised[at].bytes) return cudaSuccess;
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) return e;
-    if (at) at->bytes = bytes;
-    else raised.push_back({kernel, device, bytes});
+    if (e != cudaSuccess || at == most) return e;
+    raised[at] = {kernel, device, bytes};
+    if (at == count) ++count;
     return cudaSuccess;
 }
 

@@ -46,6 +46,8 @@ int main() {
     EXPECT(allow_dynamic_smem(one, 300000) == cudaErrorInvalidValue && calls == 7);
     std::thread([] { device = 1; sg::allow_dynamic_smem(two, 60000); }).join();
     EXPECT((limit[{(const void *)two, 1}] == 60000) && calls == 8);
+    for (device = 2; device < 100; ++device)                 // more pairs than a thread remembers
+        EXPECT(allow_dynamic_smem(one, 60000) == cudaSuccess && (limit[{(const void *)one, device}] == 60000));
     return 0;
 }
 """
