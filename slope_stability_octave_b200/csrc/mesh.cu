@@ -19,6 +19,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <new>
 
 #include "mesh.h"
@@ -168,8 +169,9 @@ static int mesh_build(sg_mesh *m, const int32_t *elem, const double *D1, const d
     // goes to block (node_i, node_j) when that lies on or above the diagonal, transposed to
     // (node_j, node_i) otherwise; the lists are filled in element order, so every block sums
     // its contributions in a fixed order
-    std::vector<int4> up_item;
-    std::vector<uint32_t> up_src;
+    std::unique_ptr<int4[]> up_item;                   // not zeroed: its pages are touched in parallel
+    std::unique_ptr<uint32_t[]> up_src;
+    int64_t n_src = 0;
     if (dim == 3 && np == 10 && n_e * 55 < ((int64_t)1 << 31)) {
         std::vector<int32_t> count(B.n_blocks, 0);
         auto each = [&](auto fn) {
@@ -187,51 +189,58 @@ static int mesh_build(sg_mesh *m, const int32_t *elem, const double *D1, const d
         // items in windows of about a hundred rows, within a window in descending number of
         // contributions: a warp's items then take the same number of loads, and what they write
         // and read stays near in time
-        std::vector<int32_t> up;
-        up.reserve((size_t)(B.n_blocks / 2 + n_n));
+        std::vector<int64_t> first(n_n + 1, 0);        // a row's first item, its first block at or right of the diagonal
+        std::vector<int32_t> diag(n_n);
+#pragma omp parallel for schedule(static)
+        for (int64_t v = 0; v < n_n; ++v) {
+            const int32_t *c0 = B.col.data() + B.row_ptr[v], *c1 = B.col.data() + B.row_ptr[v + 1];
+            diag[v] = (int32_t)(std::lower_bound(c0, c1, (int32_t)v) - B.col.data());
+            first[v + 1] = B.row_ptr[v + 1] - diag[v];
+        }
+        for (int64_t v = 0; v < n_n; ++v) first[v + 1] += first[v];
+        const int64_t nu = first[n_n], window = 1536;
+        std::vector<int32_t> up(nu);
+#pragma omp parallel for schedule(static)
         for (int64_t v = 0; v < n_n; ++v)
-            for (int32_t p = B.row_ptr[v]; p < B.row_ptr[v + 1]; ++p)
-                if (B.col[p] >= v) up.push_back(p);
-        const int64_t nu = (int64_t)up.size(), window = 1536;
+            for (int32_t p = diag[v]; p < B.row_ptr[v + 1]; ++p) up[first[v] + p - diag[v]] = p;
 #pragma omp parallel for schedule(static)
         for (int64_t u0 = 0; u0 < nu; u0 += window)
             std::stable_sort(up.begin() + u0, up.begin() + std::min(nu, u0 + window),
                              [&](int32_t a, int32_t b) { return count[a] > count[b]; });
-        std::vector<int32_t> fill(B.n_blocks, 0);
-        int32_t at = 0;
-        for (int64_t u = 0; u < nu; ++u) {
-            fill[up[u]] = at;
-            at += std::max(count[up[u]] - 4, 0);
-        }
-        std::vector<int32_t> row_of(B.n_blocks);
-        for (int64_t v = 0; v < n_n; ++v)
-            for (int32_t p = B.row_ptr[v]; p < B.row_ptr[v + 1]; ++p) row_of[p] = (int32_t)v;
-        std::vector<int32_t> item(B.n_blocks, 0);
-        up_item.resize(2 * nu);
+        std::vector<int32_t> item(B.n_blocks);         // set on and above the diagonal
+        up_item.reset(new int4[2 * nu]);
 #pragma omp parallel for schedule(static)
         for (int64_t u = 0; u < nu; ++u) {
             const int32_t p = up[u];
-            const int64_t v = row_of[p], w = B.col[p];
+            const int64_t v = std::upper_bound(B.row_ptr.begin(), B.row_ptr.end(), p) - B.row_ptr.begin() - 1, w = B.col[p];
             const int32_t *b0 = B.col.data() + B.row_ptr[w], *b1 = B.col.data() + B.row_ptr[w + 1];
             int free = 0;
             for (int c = 0; c < 3; ++c) free |= (m->Q[v * 3 + c] ? 1 << c : 0) | (m->Q[w * 3 + c] ? 8 << c : 0);
-            up_item[2 * u] = make_int4(p, (int)(std::lower_bound(b0, b1, (int32_t)v) - B.col.data()), fill[p],
+            up_item[2 * u] = make_int4(p, (int)(std::lower_bound(b0, b1, (int32_t)v) - B.col.data()), 0,
                                        count[p] | free << 24);
+            up_item[2 * u + 1] = make_int4(0, 0, 0, 0);
             item[p] = (int32_t)u;
         }
-        up_src.resize((size_t)std::max(at, 1));
+        int32_t at = 0;
+        for (int64_t u = 0; u < nu; ++u) {
+            up_item[2 * u].z = at;
+            at += std::max((up_item[2 * u].w & 0xffffff) - 4, 0);
+        }
+        n_src = std::max(at, 1);
+        up_src.reset(new uint32_t[n_src]());
         std::fill(count.begin(), count.end(), 0);     // now: contributions placed
         each([&](int32_t p, uint32_t src) {
             const int32_t c = count[p]++;
-            if (c < 4) (&up_item[2 * (int64_t)item[p] + 1].x)[c] = (int)src;
-            else up_src[fill[p] + c - 4] = src;
+            int4 *it = &up_item[2 * (int64_t)item[p]];
+            if (c < 4) (&it[1].x)[c] = (int)src;
+            else up_src[it->z + c - 4] = src;
         });
         m->n_upper = nu;
     }
 
     int rc = bsr_upload(B);
-    if (!rc && !up_src.empty()) rc = upload(&m->d_up_item, up_item.data(), up_item.size());
-    if (!rc && !up_src.empty()) rc = upload(&m->d_up_src, up_src.data(), up_src.size());
+    if (!rc && n_src) rc = upload(&m->d_up_item, up_item.get(), (size_t)(2 * m->n_upper));
+    if (!rc && n_src) rc = upload(&m->d_up_src, up_src.get(), (size_t)n_src);
     if (!rc) rc = upload(&m->d_elem, m->elem.data(), (size_t)n_e * np);
     if (!rc) rc = upload(&m->d_dphi, dphi.data(), dphi.size());
     if (!rc) rc = upload(&m->d_w, W, (size_t)n_int);
