@@ -732,7 +732,7 @@ KIND_NAMES = {
     "spmv3_f16": "k_spmv_h3 FP16 level-0 copy",
     "spmv3_f64_aorth": "k_spmv_blk 3x3 FP64 inside the A-orthogonalisation",
     "residual": "k_response3d fused stress-only residual",
-    "spmm3_f64_aorth": "k_spmm3 FP64 multi-vector SpMM of the A-orthogonalisation",
+    "spmm3_f64_aorth": "k_spmm3p / k_spmm3i FP64 multi-vector SpMM of the A-orthogonalisation (16 and 8 columns a launch)",
     "a_orthogonalize": "whole A-orthogonalisation of the deflation basis (SpMM, Gram matrix, products)",
 }
 

@@ -417,7 +417,7 @@ int sg_learned_info(const sg_learned *h, int64_t *info);
  * bracketed by CUDA events on its stream.  Kinds (capacity 12): 0 fine SpMV FP64 (FGMRES,
  * residuals), 1 fine SpMV FP32, 2 return mapping + tangent, 3 return mapping (stress),
  * 4 assembly, 5 AMG value update, 6 AMG V-cycle, 7 fine SpMV on the FP16 copy, 8 fine SpMV
- * FP64 inside sg_a_orthogonalize, 9 fused residual (sg_residual_dev), 10 fine SpMM FP64 of
+ * FP64 inside sg_a_orthogonalize, 9 fused residual (sg_residual_dev, sg_element_response_dev), 10 fine SpMM FP64 of
  * sg_a_orthogonalize (several vectors per launch), 11 a whole sg_a_orthogonalize call (units:
  * basis columns).  sg_instr_read synchronises the device and resets the
  * counters.

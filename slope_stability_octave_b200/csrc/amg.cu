@@ -783,8 +783,8 @@ template <int B, int BC> struct Team {
 // blocks of their rows and their pair indices are contiguous, so both are copied to shared memory,
 // and a pair costs one gather of P, unrolled five deep.  Runs that exceed the shared arrays are
 // halved; a single output block that does is summed from global memory.
-// What bounds it: P's sectors from L2 (39M pairs of 144 bytes: 7 TB/s).  A thread per output block, each
-// lane reading its own P block, kept the L1 tags busy instead: FP64 39M pairs 1.57 -> 1.04 ms, FP32
+// What bounds it: the L1 data pipe (82 % busy on the gathered P blocks; L2 21 %, DRAM 14 %).  A thread
+// per output block, each lane reading its own P block, kept the L1 tags busy instead: FP64 39M pairs 1.57 -> 1.04 ms, FP32
 // 4.23 -> 3.13 ms on the layered slope.  Runs of 32 or 96 blocks, or A read in place, are slower
 // (1.12 to 1.2 ms); the same form of the prolongator's A T, whose pairs read A once, gains
 // nothing in FP32.
@@ -1205,7 +1205,9 @@ __global__ void k_gjb_update(int64_t N, int64_t k0, int nb, double *__restrict__
 // tiles.  Same operations in the same order as the three kernels above.
 // What bounds it: the chain tile -> pivot inverse -> next step.  On B200 350 unknowns (11 pivot
 // blocks) took 320 us in 33 launches with the kernels above and take 140 us here (12.2 us a step; the
-// pivot block inverted by one warp's shuffles, unrolled: 25 us a step).
+// pivot block inverted by one warp's shuffles, unrolled: 25 us a step).  Whole value updates: 492 unknowns
+// 1.67 -> 1.41 ms, 876 3.22 -> 2.73, 2976 26.4 -> 26.2: past two thousand the tiles' own work is what
+// counts, and the second copy takes N^2 doubles for nothing.
 constexpr int64_t GJ_STEP_MAX = 2048;
 
 // In-place inverse of an nb x nb block held by a CTA of 256 threads, thread (r0, c) the entries

@@ -592,11 +592,11 @@ __global__ void __launch_bounds__(256) k_spmm3i(int64_t nrows, int64_t rows_per_
 // warps walk in order, so the x runs of neighbouring rows are reused from L1.
 // What bounds it: the L1 data pipe (gathers of 384 bytes a block, and two 32-bit shuffles per
 // value).  Measured on B200, 16 columns: 28.3M blocks 1.63 ms with the results written column by
-// column (1.57 + 0.13 ms with an interleaved result and an unpacking pass), 6.1M blocks 0.39 ms where
-// column-wise gathers of 8 columns took 0.52.  Tried against it: the products as FP64 MMAs with the
+// column (1.57 + 0.13 ms with an interleaved result and an unpacking pass), 6.1M blocks 0.39 ms (KEEP:
+// 0.51) where column-wise gathers of 8 columns took 0.52.  Tried against it: the products as FP64 MMAs with the
 // block row as three of eight tile rows, values straight into the fragments (2.0-2.4 ms: fewer
 // instructions, but twice the requests for the values), rows in bricks of 2 to 8 nodes a side
-// (1.67-2.0 ms: the gathers already hit L2, and its rate is not the bound).
+// (1.67-2.0 ms: the gathers already hit L2, and its rate is not the bound: L2 20 %, L1 data pipe 67 %).
 // KEEP: the two groups' products of a step are added first and join a sum that carries its
 // rounding error along (bsr_spmm_interleaved says where).  Twelve more values a lane: three
 // CTAs of 80 registers (four of 64 spill them: 1.47 against 1.22 ms for 21 columns of 6.1M blocks).
@@ -1379,7 +1379,8 @@ int gram_recurrence(int k, const double *G, double *Tp, double eps, double *Ta, 
     return SG_OK;
 }
 
-// Y(:, o) = X(:, 0:k) Ta(:, o) for o < *kout and more than 48 columns, on the FP64 tensor cores
+// Y(:, o) = X(:, 0:k) Ta(:, o) for o < *kout and more than 48 columns (the one-pass form below holds a
+// row's inputs in registers, which end there), on the FP64 tensor cores
 // (mma.sync m8n8k4 .f64, the FP64 MMA of sm_100a): CTA tile 128 rows x 64 output columns, inputs in stages of TM_MC
 // columns of X / rows of Ta staged by 8-byte cp.async (two stages, pitches padded by 4
 // doubles so the fragment reads are free of bank conflicts); warp w owns rows 32 (w & 3) ..

@@ -5,8 +5,10 @@
 //   2D: +CONSTITUTIVE_PROBLEM/mex/constitutive_2D_kernel.h:36-369
 // (elastic-perfectly plastic Mohr-Coulomb, associated flow, implicit return onto the
 // smooth face, the left / right edges or the apex; tangent from Miehe's closed form for
-// eigen-projection derivatives).  Formulas and branch tests are kept in the reference's
-// order so that the branch decision agrees with the reference's CPU code.
+// eigen-projection derivatives).  The branch tests are the reference's, in its order; what they
+// compare is written with fewer divides and sines (principal strains from one sincos, the smooth
+// face's limits multiplied out, the tangent collected by tensor), equal up to rounding, and points far
+// inside the yield surface are recognised without the principal strains.
 //
 // 3D tangent symmetry: for associated flow the tangent is exactly symmetric (every term
 // is a symmetric expression of (i, j)), so only the 21 entries with i <= j are evaluated

@@ -206,9 +206,10 @@ __device__ __forceinline__ void response_strength(const ResponseArgs &A, int64_t
 // TANGENT stores E, S and DS: a warp stages its 32 points in shared memory (odd pitch) and writes
 // contiguous runs, as k_mc3d does.
 //
-// What bounds it: latency.  The three phases of a pass depend on one another and the return
+// What bounds it: latency, with the L1 data pipe 68 % busy behind it (FP64 pipe 38 %, DRAM 24 %; with
+// the tangent 62, 23 and 45 %).  The three phases of a pass depend on one another and the return
 // mapping is a long FP64 chain, so the time goes with the passes in flight: 96-thread CTAs, eight
-// per SM at 80 registers without the tangent (a few spills cost less than the resident
+// per SM (24 warps) at 80 registers without the tangent (a few spills cost less than the resident
 // CTAs they buy: 141 us against 163 with six CTAs on the 40 m slope), four at 168 registers with
 // it (five with spills: 1.43 against 1.25 ms on the layered slope).  Measured on B200, against
 // the reduction, strain, return-mapping and force kernels in turn (stress only: the reduction and
@@ -554,8 +555,9 @@ static bool response_covers(const sg_mesh *m) {
 // Eight elements per pass of a 96-thread CTA (88 points); D, G and w come by cp.async, the next
 // pass's while B and C run; three CTAs per SM (65 KB each, registers to spare for C's 55 sums).
 //
-// What bounds it: the latency of the FP64 chains with nine warps on an SM (IPC 0.4 a scheduler,
-// FP64 pipe a quarter busy); DRAM carries DS, G and w in and 3,960 bytes an element out.  Measured on
+// What bounds it: the latency of the FP64 chains with nine warps on an SM (0.38 instructions a cycle and
+// scheduler, FP64 pipe 37 % busy, L1 data pipe 53 %); DRAM carries DS, G and w in and 3,960 bytes an
+// element out.  Measured on
 // B200 against the direct sum (k_element_blocks_p2tet_bulk): 446k points 243 -> 99 us, layered
 // slope (8.0M points) 4.06 -> 1.62 ms (3.6 TB/s).
 constexpr int EB_EL = 8, EB_THREADS = 96, EB_NQ = P2T_REF_RULE, EB_DP = 38, EB_Y = 45;
